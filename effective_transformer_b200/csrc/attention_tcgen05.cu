@@ -529,6 +529,272 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_q, const __gri
   }
 }
 
+// Sequences longer than a tile: one CTA per (sequence, 128 query rows, head), walking the sequence's keys in
+// tiles of 128 with an online softmax.  The phases of a key tile are those of the kernel above (S = Q K^T into
+// TMEM, one thread per query row, P over the scores it replaces, O_j = P V from TMEM); the running maximum, sum
+// and the 64 outputs of a row stay in its thread's registers, rescaled when the maximum moves.  K of the next
+// tile streams in under the softmax and the second MMA, V under the read of O_j and the next scores.  What
+// bounds it is that phase chain (about 7 k cycles per key tile), hidden by the four CTAs of an SM; one CTA per
+// query tile instead of one per (sequence, head) shortens the longest chain from (len / 64)^2 steps to len / 128.
+// Measured under ncu, 32 sequences of 64 to 512 tokens, 12 heads: 43 us per launch, of which the issue slots are
+// busy 42 % and the exponential unit 36 %; attention_tc_kernel, a CTA per (sequence, head): 195 us.
+// The grid is not persistent: CTAs differ by the sequence's length, and the hardware's order of starting them
+// balances that; those beyond a sequence's end leave at once.
+__global__ void __launch_bounds__(kThreads, kCtasPerSm)
+attention_tcgen05_long_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_k,
+                              const __grid_constant__ CUtensorMap tmap_v, Coords co, __half* __restrict__ ctx,
+                              const int* __restrict__ cu_seqlens, int max_tokens, int max_seq, int heads, int q_tiles,
+                              float scale_log2e, int* status_word) {
+  pdl_trigger();
+  extern __shared__ __align__(1024) uint8_t smem_raw[];
+  const uint32_t base = smem_u32(smem_raw);
+  if ((base & 1023u) != 0u) {
+    pdl_wait();  // no CTA leaves before the preceding kernel has completed
+    if (threadIdx.x == 0) report_timeout(status_word, kKernelAttnTc, kSiteSmemAlign);
+    return;
+  }
+  const uint32_t sq = base, sk = base + kTileBytes, sv = base + 2 * kTileBytes;
+  const uint32_t bar_qk = base + kBufBytes, bar_v = bar_qk + 8, bar_mma = bar_qk + 16;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem_raw + kBufBytes + 24);
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(smem_raw + kBufBytes + 32);
+  const int warp = threadIdx.x >> 5;
+  const int r = threadIdx.x;  // this thread's query row inside the tile = its TMEM lane
+
+  if (threadIdx.x == 0) {
+    mbar_init(bar_qk, 1);
+    mbar_init(bar_v, 1);
+    mbar_init(bar_mma, 1);
+    *abort_flag = 0;
+    fence_mbar_init();
+    fence_proxy_async_smem();
+    prefetch_tensormap(&tmap_q);
+    prefetch_tensormap(&tmap_k);
+    prefetch_tensormap(&tmap_v);
+  }
+  if (warp == 0) {
+    __syncwarp();
+    tmem_alloc(smem_u32(tmem_slot), kTmemCols);
+    tmem_relinquish();
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem_base = *tmem_slot;
+  const uint32_t t_lane = tmem_base + (static_cast<uint32_t>(warp * 32) << 16);
+
+  pdl_wait();  // the sequence bounds and the Q/K/V rows come from earlier kernels
+  const int head = blockIdx.x % heads, tile = blockIdx.x / heads;
+  const int b = tile / q_tiles, q0 = (tile - b * q_tiles) * kTileRows;
+  const int first = max(cu_seqlens[b], 0);
+  const int len = min(min(cu_seqlens[b + 1], max_tokens) - first, max_seq);
+  if (q0 < len) {  // uniform in the CTA
+    const int nq = min(kTileRows, len - q0);
+    const int k_tiles = (len + kTileRows - 1) / kTileRows;
+    const int x = head * co.x_per_head, y = head * co.y_per_head + first;
+    auto boxes_of = [&](int row0) { return (min(kTileRows, len - row0) + kBoxRows - 1) / kBoxRows; };
+    auto load_rows = [&](uint32_t dst, const CUtensorMap* map, int row0, int boxes, uint32_t bar) {
+      for (int j = 0; j < boxes; ++j) tma_load_2d(dst + j * kBoxBytes, map, x, y + row0 + j * kBoxRows, bar);
+    };
+    auto wait_all = [&](uint32_t bar, uint32_t phase, int site) {
+      const bool got = mbar_wait(bar, phase, abort_flag);
+      if (!got) {
+        *abort_flag = 1;
+        report_timeout(status_word, kKernelAttnTc, site);
+      }
+      return __syncthreads_and(got) != 0;
+    };
+    int qk_issued = 0, v_issued = 0, qk_seen = 0, v_seen = 0;  // copies requested / waited for
+    if (threadIdx.x == 0) {
+      const int bq = boxes_of(q0), bk = boxes_of(0);
+      mbar_arrive_expect_tx(bar_qk, static_cast<uint32_t>((bq + bk) * kBoxBytes));
+      load_rows(sq, &tmap_q, q0, bq, bar_qk);
+      load_rows(sk, &tmap_k, 0, bk, bar_qk);
+      mbar_arrive_expect_tx(bar_v, static_cast<uint32_t>(bk * kBoxBytes));
+      load_rows(sv, &tmap_v, 0, bk, bar_v);
+    }
+    qk_issued = v_issued = 1;
+
+    const bool warp_has_rows = warp * 32 < nq;
+    float o[kD];
+#pragma unroll
+    for (int e = 0; e < kD; ++e) o[e] = 0.f;
+    float m = -INFINITY, l = 0.f;
+    uint32_t mma_phase = 0;
+    bool ok = true;
+    for (int j = 0; j < k_tiles && ok; ++j) {
+      const int n = min(kTileRows, len - j * kTileRows);
+      const int n16 = (n + 15) & ~15;
+      const bool has_next = j + 1 < k_tiles;
+      ok = wait_all(bar_qk, static_cast<uint32_t>(j & 1), kSiteLoad);
+      if (!ok) break;
+      ++qk_seen;
+      // ---- S = Q K^T ----
+      if (threadIdx.x == 0) {
+        tc_fence_after();
+        const uint32_t idesc = idesc_f16(kTileRows, n16, false);
+        const uint64_t qd = make_kmajor_sw128_desc(sq), kd = make_kmajor_sw128_desc(sk);
+#pragma unroll
+        for (int k = 0; k < kD / 16; ++k) umma_f16_ss(tmem_base, qd + 2u * k, kd + 2u * k, idesc, k != 0 ? 1u : 0u);
+        umma_commit(bar_mma);
+      }
+      ok = wait_all(bar_mma, mma_phase, kSiteScores);
+      mma_phase ^= 1u;
+      if (!ok) break;
+      tc_fence_after();
+      if (has_next) {  // K is dead
+        if (threadIdx.x == 0) {
+          const int bk = boxes_of((j + 1) * kTileRows);
+          mbar_arrive_expect_tx(bar_qk, static_cast<uint32_t>(bk * kBoxBytes));
+          load_rows(sk, &tmap_k, (j + 1) * kTileRows, bk, bar_qk);
+        }
+        ++qk_issued;
+      }
+      float corr = 1.f;
+      if (warp_has_rows) {
+        float m2[2] = {m, -INFINITY};
+        for (int c0 = 0; c0 < n; c0 += 32) {
+          uint32_t s32[32];
+          tmem_ld_32x32b_x32(t_lane + c0, s32);
+          tmem_ld_wait();
+          if (c0 + 32 <= n) {
+#pragma unroll
+            for (int e = 0; e < 32; ++e) m2[e & 1] = fmaxf(m2[e & 1], __uint_as_float(s32[e]));
+          } else {
+#pragma unroll
+            for (int e = 0; e < 32; ++e)
+              if (c0 + e < n) m2[e & 1] = fmaxf(m2[e & 1], __uint_as_float(s32[e]));
+          }
+        }
+        const float m_new = fmaxf(m2[0], m2[1]);
+        corr = ex2_approx((m - m_new) * scale_log2e);  // 0 for the first tile (m = -inf)
+        m = m_new;
+        const float ms = -m * scale_log2e;
+        float l2[2] = {l * corr, 0.f};
+        for (int c0 = 0; c0 < n16; c0 += 32) {
+          uint32_t s32[32], pk[16];
+          tmem_ld_32x32b_x32(t_lane + c0, s32);
+          tmem_ld_wait();
+          if (c0 + 32 <= n) {
+#pragma unroll
+            for (int e = 0; e < 16; ++e) {
+              const float p0 = ex2_approx(fmaf(__uint_as_float(s32[2 * e]), scale_log2e, ms));
+              const float p1 = ex2_approx(fmaf(__uint_as_float(s32[2 * e + 1]), scale_log2e, ms));
+              l2[0] += p0;
+              l2[1] += p1;
+              pk[e] = pack_half2(p0, p1);
+            }
+          } else {
+            // columns past the sequence (stale or another sequence's scores) weigh nothing
+#pragma unroll
+            for (int e = 0; e < 16; ++e) {
+              const float p0 = c0 + 2 * e < n ? ex2_approx(fmaf(__uint_as_float(s32[2 * e]), scale_log2e, ms)) : 0.f;
+              const float p1 =
+                  c0 + 2 * e + 1 < n ? ex2_approx(fmaf(__uint_as_float(s32[2 * e + 1]), scale_log2e, ms)) : 0.f;
+              l2[0] += p0;
+              l2[1] += p1;
+              pk[e] = pack_half2(p0, p1);
+            }
+          }
+          // 32 keys = 16 packed columns, over score columns this thread has already read
+          tmem_st_32x32b_x16(t_lane + kPCol + (c0 >> 1), pk);
+        }
+        l = l2[0] + l2[1];
+        tmem_st_wait();
+      }
+      // V rows [n, n16) belong to another sequence or are stale: P is zero there, so make V finite there too
+      const bool got_v = mbar_wait(bar_v, static_cast<uint32_t>(j & 1), abort_flag);
+      if (!got_v) {
+        *abort_flag = 1;
+        report_timeout(status_word, kKernelAttnTc, kSiteLoad);
+      }
+      for (int idx = threadIdx.x; idx < (n16 - n) * 8; idx += kThreads)
+        st_shared_v4(sv + (n + (idx >> 3)) * 128 + ((idx & 7) << 4), 0u, 0u, 0u, 0u);
+      fence_proxy_async_smem();
+      tc_fence_before();
+      ok = __syncthreads_and(got_v) != 0;
+      if (!ok) break;
+      ++v_seen;
+      // ---- O_j = P V ----
+      if (threadIdx.x == 0) {
+        tc_fence_after();
+        const uint32_t idesc = idesc_f16(kTileRows, kD, true);
+        for (int ks = 0; ks < n16 / 16; ++ks) {
+          const uint64_t vd = make_kmajor_sw128_desc(sv + ks * 2048);  // MN-major: 16 keys = two 8-row groups
+          umma_f16_ts(tmem_base + kOCol, tmem_base + kPCol + ks * 8, vd, idesc, ks != 0 ? 1u : 0u);
+        }
+        umma_commit(bar_mma);
+      }
+      ok = wait_all(bar_mma, mma_phase, kSiteContext);
+      mma_phase ^= 1u;
+      if (!ok) break;
+      tc_fence_after();
+      if (has_next) {  // V is dead
+        if (threadIdx.x == 0) {
+          fence_proxy_async_smem();
+          const int bk = boxes_of((j + 1) * kTileRows);
+          mbar_arrive_expect_tx(bar_v, static_cast<uint32_t>(bk * kBoxBytes));
+          load_rows(sv, &tmap_v, (j + 1) * kTileRows, bk, bar_v);
+        }
+        ++v_issued;
+      }
+      if (warp_has_rows) {
+#pragma unroll
+        for (int h = 0; h < kD; h += 16) {
+          uint32_t ov[16];
+          tmem_ld_32x32b_x16(t_lane + kOCol + h, ov);
+          tmem_ld_wait();
+#pragma unroll
+          for (int e = 0; e < 16; ++e) o[h + e] = fmaf(o[h + e], corr, __uint_as_float(ov[e]));
+        }
+      }
+      tc_fence_before();  // ordered before the next scores by the barrier in the wait for K
+    }
+    if (warp_has_rows && ok && r < nq) {
+      const float inv_l = 1.0f / l;
+      __half* op = ctx + static_cast<size_t>(first + q0 + r) * (heads * kD) + head * kD;
+#pragma unroll
+      for (int q4 = 0; q4 < 4; ++q4) {
+        uint32_t w[8];
+#pragma unroll
+        for (int e = 0; e < 8; ++e) w[e] = pack_half2(o[q4 * 16 + 2 * e] * inv_l, o[q4 * 16 + 2 * e + 1] * inv_l);
+        asm volatile("st.global.v8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"l"(op + q4 * 16), "r"(w[0]), "r"(w[1]),
+                     "r"(w[2]), "r"(w[3]), "r"(w[4]), "r"(w[5]), "r"(w[6]), "r"(w[7])
+                     : "memory");
+      }
+    }
+    if (threadIdx.x == 0 && !ok) {  // copies in flight must land before the shared memory goes away
+      if (qk_issued > qk_seen) mbar_wait(bar_qk, static_cast<uint32_t>((qk_issued - 1) & 1), abort_flag);
+      if (v_issued > v_seen) mbar_wait(bar_v, static_cast<uint32_t>((v_issued - 1) & 1), abort_flag);
+    }
+  }
+
+  tc_fence_before();
+  __syncthreads();
+  if (warp == 0) {
+    __syncwarp();
+    tc_fence_after();
+    tmem_dealloc(tmem_base, kTmemCols);
+  }
+}
+
+// How (token, head) maps to TMA coordinates, and the extent of the tensor they index.
+bool qkv_coords(long long token_stride, long long head_stride, int heads, int max_tokens, Coords* co, uint64_t* cols,
+                uint64_t* rows) {
+  if (static_cast<long long>(heads - 1) * head_stride + kD <= token_stride) {
+    *co = {static_cast<int>(head_stride), 0};
+    *cols = static_cast<uint64_t>(heads - 1) * head_stride + kD;
+    *rows = static_cast<uint64_t>(max_tokens);
+    return true;
+  }
+  if (token_stride == kD && head_stride % token_stride == 0 && head_stride / token_stride >= max_tokens) {
+    *co = {0, static_cast<int>(head_stride / token_stride)};
+    *cols = kD;
+    *rows = static_cast<uint64_t>(heads - 1) * (head_stride / token_stride) + max_tokens;
+    return true;
+  }
+  return false;
+}
+
 }  // namespace
 
 size_t attention_plan_ints(int batch, int max_tokens) { return plan_ints(batch, max_tokens); }
@@ -555,17 +821,7 @@ cudaError_t launch_attention_tcgen05(const __half* q, const __half* k, const __h
     return cudaErrorMisalignedAddress;
   Coords co;
   uint64_t cols, rows;
-  if (static_cast<long long>(heads - 1) * head_stride + kD <= token_stride) {
-    co = {static_cast<int>(head_stride), 0};
-    cols = static_cast<uint64_t>(heads - 1) * head_stride + kD;
-    rows = static_cast<uint64_t>(max_tokens);
-  } else if (token_stride == kD && head_stride % token_stride == 0 && head_stride / token_stride >= max_tokens) {
-    co = {0, static_cast<int>(head_stride / token_stride)};
-    cols = kD;
-    rows = static_cast<uint64_t>(heads - 1) * (head_stride / token_stride) + max_tokens;
-  } else {
-    return cudaErrorInvalidValue;
-  }
+  if (!qkv_coords(token_stride, head_stride, heads, max_tokens, &co, &cols, &rows)) return cudaErrorInvalidValue;
   CUtensorMap tq, tk, tv;
   if (!encode_2d_fp16_sw128(&tq, q, rows, cols, static_cast<uint64_t>(token_stride), kBoxRows, kD, maps) ||
       !encode_2d_fp16_sw128(&tk, k, rows, cols, static_cast<uint64_t>(token_stride), kBoxRows, kD, maps) ||
@@ -596,6 +852,41 @@ cudaError_t launch_attention_tcgen05(const __half* q, const __half* k, const __h
                 : launch_pdl(attention_tcgen05_kernel<false>, dim3(static_cast<int>(grid)), dim3(kThreads), kSmemBytes,
                              stream, tq, tk, tv, co, ctx, plan, batch, max_tokens, heads, scale_log2e, status_word,
                              reverse ? 1 : 0, ma);
+}
+
+bool attention_long_supported(const __half* ctx, int max_seq) {
+  return max_seq > kTileRows && (reinterpret_cast<uintptr_t>(ctx) & 31u) == 0;
+}
+
+cudaError_t launch_attention_tcgen05_long(const __half* q, const __half* k, const __half* v, long long token_stride,
+                                          long long head_stride, __half* ctx, const int* cu_seqlens, int batch,
+                                          int max_seq, int max_tokens, int heads, int d, int* status_word,
+                                          cudaStream_t stream, TensorMapCache* maps) {
+  if (batch <= 0 || heads <= 0 || max_tokens <= 0 || max_seq <= 0) return cudaSuccess;
+  if (d != kD || token_stride < kD || (token_stride % 8) != 0 || (head_stride % 8) != 0 || head_stride < 0)
+    return cudaErrorInvalidValue;
+  if (((reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(k) | reinterpret_cast<uintptr_t>(v)) & 15u) ||
+      (reinterpret_cast<uintptr_t>(ctx) & 31u))
+    return cudaErrorMisalignedAddress;
+  Coords co;
+  uint64_t cols, rows;
+  if (!qkv_coords(token_stride, head_stride, heads, max_tokens, &co, &cols, &rows)) return cudaErrorInvalidValue;
+  CUtensorMap tq, tk, tv;
+  if (!encode_2d_fp16_sw128(&tq, q, rows, cols, static_cast<uint64_t>(token_stride), kBoxRows, kD, maps) ||
+      !encode_2d_fp16_sw128(&tk, k, rows, cols, static_cast<uint64_t>(token_stride), kBoxRows, kD, maps) ||
+      !encode_2d_fp16_sw128(&tv, v, rows, cols, static_cast<uint64_t>(token_stride), kBoxRows, kD, maps))
+    return cudaErrorInvalidValue;
+  static PerDeviceOnce once;  // function attributes are per device
+  const cudaError_t once_err = once.run([] {
+    return cudaFuncSetAttribute(attention_tcgen05_long_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes);
+  });
+  if (once_err != cudaSuccess) return once_err;
+  const int q_tiles = (min(max_seq, max_tokens) + kTileRows - 1) / kTileRows;
+  const long long grid = static_cast<long long>(batch) * q_tiles * heads;
+  if (grid > 0x7fffffffLL) return cudaErrorInvalidValue;
+  const float scale_log2e = (1.0f / sqrtf(static_cast<float>(d))) * 1.4426950408889634f;
+  return launch_pdl(attention_tcgen05_long_kernel, dim3(static_cast<unsigned>(grid)), dim3(kThreads), kSmemBytes, stream,
+                    tq, tk, tv, co, ctx, cu_seqlens, max_tokens, max_seq, heads, q_tiles, scale_log2e, status_word);
 }
 
 }  // namespace etb

@@ -365,6 +365,13 @@ cudaError_t launch_attention_tc(const __half* q, const __half* k, const __half* 
                                 long long token_stride, long long head_stride, __half* ctx,
                                 const int* cu_seqlens, int batch, int max_seq, int max_tokens, int heads,
                                 int d, int* status_word, cudaStream_t stream, TensorMapCache* maps = nullptr);
+// tcgen05 attention for batches with sequences longer than 128 tokens (attention_long_supported: any
+// shorter ones in the batch are served too; the context on a 32-byte boundary); arguments as above.
+bool attention_long_supported(const __half* ctx, int max_seq);
+cudaError_t launch_attention_tcgen05_long(const __half* q, const __half* k, const __half* v, long long token_stride,
+                                          long long head_stride, __half* ctx, const int* cu_seqlens, int batch,
+                                          int max_seq, int max_tokens, int heads, int d, int* status_word,
+                                          cudaStream_t stream, TensorMapCache* maps = nullptr);
 // tcgen05 attention for sequences of at most 128 tokens: a plan (sequences
 // packed into 128-row tiles) made once per batch, then one launch per layer.
 // attr_mask given ([B, seq, seq], 1 = attend; with batch_idx / word_idx of the packed rows): a

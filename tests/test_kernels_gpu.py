@@ -276,6 +276,17 @@ def test_attention_tensor_core(lens, layout):
     _attention_case(torch.float16, lens, 2, use_simt=False, layout=layout)
 
 
+# more than one 128-row query or key tile: one row past a tile, whole tiles, short and empty sequences between
+# long ones, BERT's 512 positions and beyond
+LONG_LEN_CASES = [[129], [256], [257, 1, 512, 0, 255], [130, 384, 16, 17, 500], [1000, 128, 127]]
+
+
+@pytest.mark.parametrize("lens", LONG_LEN_CASES)
+@pytest.mark.parametrize("layout", ["qkv", "headmajor"])
+def test_attention_tcgen05_sequences_longer_than_a_tile(lens, layout):
+    _attention_case(torch.float16, lens, 12 if sum(lens) < 600 else 2, use_simt=False, layout=layout)
+
+
 @pytest.mark.parametrize("lens", LEN_CASES)
 @pytest.mark.parametrize("layout", ["qkv", "headmajor", "unaligned"])
 def test_attention_fp32_on_tensor_cores_keeps_fp32_accuracy(lens, layout):
