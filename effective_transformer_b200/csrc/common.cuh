@@ -394,17 +394,40 @@ cudaError_t launch_split_tf32(const float* x, float* hi, float* lo, const int* r
 cudaError_t launch_gemm_tf32x3(const float* a_hi, const float* a_lo, const float* w_hi, const float* w_lo,
                                const float* bias, float* c, const int* m_ptr, int max_m, int n, int k,
                                int epilogue, int* status_word, cudaStream_t stream, bool reverse_m = false,
-                               float* c_lo = nullptr, TensorMapCache* maps = nullptr);
+                               float* c_lo = nullptr, TensorMapCache* maps = nullptr, bool weights_ready = false);
 // tcgen05 GEMM, fp16 in / fp32 accumulate / fp16 out.  w_packed is [N,K].
 // reverse_m: row tiles are visited from the last to the first.  A kernel that
 // consumes what the previous kernel has just written finds the rows written
 // last still in L2 if it starts with them, so consecutive kernels of a layer
 // alternate their direction.
+// weights_ready: w_packed was complete before the preceding kernel of the stream began (the handle's own
+// weights), so a kernel may fetch it before it waits for that kernel.
 cudaError_t launch_gemm_tcgen05(const __half* a, const __half* w_packed, const __half* bias,
                                 __half* c, const int* m_ptr, int max_m, int n, int k, int epilogue,
                                 int* status_word, cudaStream_t stream, bool reverse_m = false,
                                 const __half* residual = nullptr, TensorMapCache* maps = nullptr,
-                                const GemmLayerNorm* ln = nullptr);
+                                const GemmLayerNorm* ln = nullptr, bool weights_ready = false);
+// Projections of small batches on tiles of 128 x 64 whose K range is split over a cluster
+// (gemm_split.cu).  fp16: a [max_m,k], w [n,k], c fp16.  a_lo / w_lo given: fp32 by the three-product tf32
+// split, c_lo as in launch_gemm_tf32x3.
+struct SplitGemm {
+  const void* a = nullptr;
+  const void* a_lo = nullptr;
+  const void* w = nullptr;
+  const void* w_lo = nullptr;
+  const void* bias = nullptr;
+  const void* residual = nullptr;
+  void* c = nullptr;
+  float* c_lo = nullptr;
+  const int* m_ptr = nullptr;
+  int max_m = 0, n = 0, k = 0;
+  bool weights_ready = false;  // w was complete before the preceding kernel of the stream began
+  int* status_word = nullptr;
+  GemmLayerNorm ln;
+};
+// How many CTAs share a tile's K range, or 0 where the persistent kernels serve the shape better.
+int gemm_split_count(int max_m, int n, int k, bool tf32);
+cudaError_t launch_gemm_split(const SplitGemm& g, int epilogue, int splits, TensorMapCache* maps, cudaStream_t stream);
 // Whether the fused LayerNorm epilogues can serve a projection of n output columns.
 inline bool gemm_layernorm_supported(int n) { return n > 0 && n % 256 == 0 && n <= 1024; }
 

@@ -457,7 +457,7 @@ int run_layer(et_handle_t h, const LayerWeights& lw, const T* x_in, T* x_out, co
     if (tc)
       return launch_gemm_tcgen05(reinterpret_cast<const __half*>(a), static_cast<const __half*>(w_t),
                                  static_cast<const __half*>(bias), reinterpret_cast<__half*>(c), t_ptr,
-                                 max_m, n, k, epi, ws.status, s, turn(), nullptr, &h->maps);
+                                 max_m, n, k, epi, ws.status, s, turn(), nullptr, &h->maps, nullptr, true);
     if (tc32) {
       // w_t holds rn_tf32(W), w_lo the remainder; the input is split the same way first
       const float* a_hi = reinterpret_cast<const float*>(a);
@@ -470,7 +470,7 @@ int run_layer(et_handle_t h, const LayerWeights& lw, const T* x_in, T* x_out, co
       }
       return launch_gemm_tf32x3(a_hi, a_lo, static_cast<const float*>(w_t), static_cast<const float*>(w_lo),
                                 static_cast<const float*>(bias), reinterpret_cast<float*>(c), t_ptr, max_m, n, k,
-                                epi, ws.status, s, turn(), c_lo, &h->maps);
+                                epi, ws.status, s, turn(), c_lo, &h->maps, true);
     }
     forward_only();
     return launch_gemm_simt<T>(a, B(w_rm), B(bias), c, t_ptr, max_m, n, k, epi, s);
@@ -493,7 +493,7 @@ int run_layer(et_handle_t h, const LayerWeights& lw, const T* x_in, T* x_out, co
     nin.csum = H16(lw.cqkv);
     ET_LAUNCH(h, ET_PROF_GEMM_QKV, 1, s,
               launch_gemm_tcgen05(H16(x_in), H16(lw.wqkv_f), H16(lw.bqkv_f), reinterpret_cast<__half*>(qkv), t_ptr,
-                                  max_m, 3 * hid, hid, kEpiNormIn, ws.status, s, turn(), nullptr, &h->maps, &nin));
+                                  max_m, 3 * hid, hid, kEpiNormIn, ws.status, s, turn(), nullptr, &h->maps, &nin, true));
   } else if (tc32 && in_split_ready)
     ET_LAUNCH(h, ET_PROF_GEMM_QKV, 1, s,
               gemm(reinterpret_cast<const T*>(ws.a_hi), lw.wqkv, lw.wqkv_t, lw.wqkv_lo, lw.bqkv, qkv, 3 * hid, hid,
@@ -558,7 +558,7 @@ int run_layer(et_handle_t h, const LayerWeights& lw, const T* x_in, T* x_out, co
     n1.stats_out = ws.stats_att;
     ET_LAUNCH(h, ET_PROF_GEMM_ATTN_OUT, 1, s,
               launch_gemm_tcgen05(H16(ctx), H16(lw.wo_t), H16(lw.bo), reinterpret_cast<__half*>(att), t_ptr, max_m,
-                                  hid, hid, kEpiNormResidual, ws.status, s, turn(), H16(x_in), &h->maps, &n1));
+                                  hid, hid, kEpiNormResidual, ws.status, s, turn(), H16(x_in), &h->maps, &n1, true));
     // first feed-forward projection of LN1(att): folded weights, statistics, GELU
     GemmLayerNorm n2;
     n2.eps = h->eps;
@@ -567,7 +567,7 @@ int run_layer(et_handle_t h, const LayerWeights& lw, const T* x_in, T* x_out, co
     n2.csum = H16(lw.c1);
     ET_LAUNCH(h, ET_PROF_GEMM_FFN1, 1, s,
               launch_gemm_tcgen05(H16(att), H16(lw.w1_f), H16(lw.b1_f), reinterpret_cast<__half*>(ffn), t_ptr, max_m,
-                                  f, hid, kEpiNormInGelu, ws.status, s, turn(), nullptr, &h->maps, &n2));
+                                  f, hid, kEpiNormInGelu, ws.status, s, turn(), nullptr, &h->maps, &n2, true));
     // second: + bias + LN1(att) on the fly; leaves the sum in x_out and its statistics in ws.stats_x
     GemmLayerNorm n3;
     n3.eps = h->eps;
@@ -578,7 +578,7 @@ int run_layer(et_handle_t h, const LayerWeights& lw, const T* x_in, T* x_out, co
     n3.stats_out = ws.stats_x;
     ET_LAUNCH(h, ET_PROF_GEMM_FFN2, 1, s,
               launch_gemm_tcgen05(H16(ffn), H16(lw.w2_t), H16(lw.b2), reinterpret_cast<__half*>(x_out), t_ptr, max_m,
-                                  hid, f, kEpiNormResidual, ws.status, s, turn(), H16(att), &h->maps, &n3));
+                                  hid, f, kEpiNormResidual, ws.status, s, turn(), H16(att), &h->maps, &n3, true));
     return ET_OK;
   }
   const bool ln_in_gemm = tc && h->fuse_ln && gemm_layernorm_supported(hid);
@@ -621,7 +621,7 @@ int run_layer(et_handle_t h, const LayerWeights& lw, const T* x_in, T* x_out, co
   } else if (tc) {
     ET_LAUNCH(h, ET_PROF_GEMM_FFN2, 1, s,
               launch_gemm_tcgen05(H16(ffn), H16(lw.w2_t), H16(lw.b2), reinterpret_cast<__half*>(x_out), t_ptr, max_m,
-                                  hid, f, kEpiBiasResidual, ws.status, s, turn(), H16(att), &h->maps));
+                                  hid, f, kEpiBiasResidual, ws.status, s, turn(), H16(att), &h->maps, nullptr, true));
     ET_LAUNCH(h, ET_PROF_LAYERNORM, 1, s,
               launch_add_bias_input_layernorm<T>(x_out, nullptr, nullptr, B(lw.ln2_gamma), B(lw.ln2_beta), t_ptr,
                                                  max_m, hid, h->eps, s, turn()));
@@ -801,7 +801,7 @@ int pooler_impl(et_handle_t h, const void* packed, const int* cu_seqlens, void* 
     ET_LAUNCH(h, ET_PROF_POOLER, 1, s,
               launch_gemm_tcgen05(static_cast<const __half*>(ws.first_tok), static_cast<const __half*>(mw.pool_w_t),
                                   static_cast<const __half*>(mw.pool_b), static_cast<__half*>(pooled_out),
-                                  ws.pool_m, batch, hid, hid, kEpiBiasTanh, ws.status, s, false, nullptr, &h->maps));
+                                  ws.pool_m, batch, hid, hid, kEpiBiasTanh, ws.status, s, false, nullptr, &h->maps, nullptr, true));
   else if (h->cfg.dtype == ET_FP16)
     ET_LAUNCH(h, ET_PROF_POOLER, 1, s,
               launch_gemm_simt<__half>(static_cast<const __half*>(ws.first_tok), static_cast<const __half*>(mw.pool_w),

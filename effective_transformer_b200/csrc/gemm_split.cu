@@ -1,0 +1,571 @@
+// Projections of small batches: C[M,N] = epilogue(A[M,K] * W[N,K]^T), the K range of a tile split over
+// the CTAs of a cluster.
+//
+// The persistent kernels (gemm_tcgen05.cu, gemm_tf32x3.cu) give a CTA (pair) whole 256-wide tiles with all
+// of K: right when there are tiles for every SM, but a batch of a few hundred tokens has 3 to 24 of them,
+// and each walks K alone (48 dependent 64-wide steps for K = 3072) while most of the GPU idles.  What
+// bounds such a projection is the latency of that chain and how many SMs pull on the weights (1 to 5 MB).
+// So here a tile is 128 x 64 and its K range is cut into `splits` (1, 2, 4 or 8) parts, one CTA each:
+//   warp 0      TMA producer: A [128 x BK] and W [64 x BK] boxes into a ring of shared-memory stages
+//   warp 1      tcgen05.mma (M = 128, N = 64) into TMEM, one accumulator block per accumulation unit
+//   warps 2-5   read the partial sums from TMEM and send row r to the CTA r % splits of the cluster through
+//               distributed shared memory; behind a cluster barrier each CTA adds the parts of its rows
+//               in rank order (the result does not depend on timing), applies the epilogue and stores
+// Rows are dealt to the CTAs by r % splits, so a last tile with few rows still keeps all of them busy.
+// The shared memory of a CTA is below half an SM's, so the next projection's CTAs are resident while this
+// one runs, and the producer requests their W boxes before it waits for this kernel
+// (`weights_ready`: W was complete before the preceding kernel began): a weight's trip from HBM then lies
+// under the kernel before.  Every mbarrier wait is bounded.
+#include "common.cuh"
+#include "ptx_sm100.cuh"
+
+#include <type_traits>
+
+namespace etb {
+
+namespace {
+
+using namespace ptx;
+
+constexpr int BM = 128;
+constexpr int BN = 64;
+constexpr int kRowBytes = 128;        // one swizzle row of an operand tile: 64 fp16 or 32 tf32
+constexpr int kThreads = 192;
+constexpr int kEpThreads = 128;
+constexpr int kMaxSplits = 8;
+
+enum Site : int { kSiteProducer = 1, kSiteDrain = 2, kSiteMma = 3, kSiteMmaDrain = 4, kSiteEpilogue = 5, kSiteAlign = 6 };
+
+template <bool kTf32>
+struct Cfg {
+  static constexpr int BK = kTf32 ? 32 : 64;
+  static constexpr int kParts = kTf32 ? 2 : 1;  // tf32: hi and lo halves of both operands
+  static constexpr int kABytes = BM * kRowBytes;
+  static constexpr int kWBytes = BN * kRowBytes;
+  static constexpr int kStageBytes = kParts * (kABytes + kWBytes);
+  static constexpr int kStages = 3;
+  // tf32: the tensor core adds into its accumulator with truncation, so a chain is cut every six k-blocks
+  // (see gemm_tf32x3.cu); every unit has a TMEM block of its own here.  fp16: one unit.
+  static constexpr int kUnitKb = kTf32 ? 6 : 1 << 20;
+  static constexpr int kBlocks = kTf32 ? 8 : 1;
+  static constexpr int kTmemCols = kBlocks * BN;
+  static constexpr int kRecvBytes = BM * BN * 4;
+  static constexpr int kNumBars = 2 * kStages + 2;
+  static constexpr int kSmemBytes = kStages * kStageBytes + kRecvBytes + 128;
+};
+
+__device__ __forceinline__ void umma_tf32_ss(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
+                                             uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::1.kind::tf32 [%0], %1, %2, %3, p;\n\t}"
+      ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
+      : "memory");
+}
+__device__ __forceinline__ void st_cluster_v4(uint32_t addr, float a, float b, float c, float d) {
+  asm volatile("st.shared::cluster.v4.f32 [%0], {%1,%2,%3,%4};" ::"r"(addr), "f"(a), "f"(b), "f"(c), "f"(d)
+               : "memory");
+}
+__device__ __forceinline__ float4 ld_shared_f4(uint32_t addr) {
+  float4 v;
+  asm volatile("ld.shared.v4.f32 {%0,%1,%2,%3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(addr) : "memory");
+  return v;
+}
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
+
+__device__ __forceinline__ uint32_t gelu_tanh_half2(uint32_t xbits) {  // as in gemm_tcgen05.cu
+  const __half2 x = *reinterpret_cast<const __half2*>(&xbits);
+  const __half2 c1 = __float2half2_rn(0.7978845608028654f);
+  const __half2 c2 = __float2half2_rn(0.7978845608028654f * 0.044715f);
+  const __half2 u = __hmul2(x, __hfma2(__hmul2(x, x), c2, c1));
+  const uint32_t ubits = *reinterpret_cast<const uint32_t*>(&u);
+  uint32_t tbits;
+  asm("tanh.approx.f16x2 %0, %1;" : "=r"(tbits) : "r"(ubits));
+  const __half2 th = *reinterpret_cast<const __half2*>(&tbits);
+  const __half2 hx = __hmul2(x, __float2half2_rn(0.5f));
+  const __half2 y = __hfma2(hx, th, hx);
+  return *reinterpret_cast<const uint32_t*>(&y);
+}
+
+__device__ __forceinline__ void load8(const __half* p, float* f) { VecTraits<__half>::unpack(ld_global_nc_v4(p), f); }
+__device__ __forceinline__ void load8(const float* p, float* f) {
+  VecTraits<float>::unpack(ld_global_nc_v4(p), f);
+  VecTraits<float>::unpack(ld_global_nc_v4(p + 4), f + 4);
+}
+
+struct Maps {
+  CUtensorMap a, w, a_lo, w_lo;  // the lo halves only for tf32
+};
+
+template <bool kTf32, int EPI>
+__global__ void __launch_bounds__(kThreads, kTf32 ? 1 : 2)
+gemm_split_kernel(const __grid_constant__ Maps maps, void* __restrict__ c_ptr, float* __restrict__ c_lo,
+                  const void* __restrict__ bias_ptr, const void* __restrict__ res_ptr, const int* __restrict__ m_ptr,
+                  int max_m, int N, int num_kb, int weights_ready, int* status_word, const GemmLayerNorm ln) {
+  using cfg = Cfg<kTf32>;
+  using T = typename std::conditional<kTf32, float, __half>::type;
+  constexpr int S = cfg::kStages;
+  constexpr bool kNormIn = EPI == kEpiNormIn || EPI == kEpiNormInGelu;
+  constexpr bool kResidual = EPI == kEpiBiasResidual || EPI == kEpiNormResidual;
+
+  pdl_trigger();
+  const int splits = gridDim.x, rank = blockIdx.x;  // the cluster covers gridDim.x
+  const int m0 = blockIdx.z * BM, n0 = blockIdx.y * BN;
+  const int kb0 = num_kb * rank / splits, kb1 = num_kb * (rank + 1) / splits;
+  const int units = (kb1 - kb0 + cfg::kUnitKb - 1) / cfg::kUnitKb;
+
+  extern __shared__ __align__(1024) uint8_t smem_raw[];
+  const uint32_t base = smem_u32(smem_raw);
+  const bool aligned = (base & 1023u) == 0u;  // the same in every CTA of the grid
+  const uint32_t recv = base + S * cfg::kStageBytes;
+  const uint32_t bar0 = recv + cfg::kRecvBytes;
+  auto full_bar = [&](int s) { return bar0 + 8u * s; };
+  auto empty_bar = [&](int s) { return bar0 + 8u * (S + s); };
+  const uint32_t acc_bar = bar0 + 8u * (2 * S), drain_bar = acc_bar + 8u;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem_raw + S * cfg::kStageBytes + cfg::kRecvBytes + 8 * cfg::kNumBars);
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < S; ++s) {
+      mbar_init(full_bar(s), 1);
+      mbar_init(empty_bar(s), 1);
+    }
+    mbar_init(acc_bar, 1);
+    mbar_init(drain_bar, 1);
+    *abort_flag = 0;
+    fence_mbar_init();
+    fence_proxy_async_smem();
+  }
+  if (warp == 1) {
+    tmem_alloc(smem_u32(tmem_slot), cfg::kTmemCols);
+    tmem_relinquish();
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem_base = *tmem_slot;
+  // every CTA of the cluster runs from here on: its shared memory may be written once all have arrived
+  if (splits > 1) cluster_arrive();
+
+  auto fail = [&](int site) {
+    *abort_flag = 1;
+    report_timeout(status_word, kKernelGemmTc, 16 + site);
+  };
+  auto valid_rows = [&]() {
+    const int M = *m_ptr;
+    return (M < 0 ? 0 : (M > max_m ? max_m : M)) - m0;  // of this tile, <= 0: nothing to do
+  };
+
+  if (warp == 0) {
+    // ------------------------- TMA producer -------------------------
+    if (lane == 0 && aligned) {
+      const CUtensorMap* map_a[2] = {&maps.a, &maps.a_lo};
+      const CUtensorMap* map_w[2] = {&maps.w, &maps.w_lo};
+      auto load_w = [&](int kb, int s) {
+        mbar_arrive_expect_tx(full_bar(s), cfg::kStageBytes);
+        const uint32_t dst = base + s * cfg::kStageBytes + cfg::kParts * cfg::kABytes;
+#pragma unroll
+        for (int h = 0; h < cfg::kParts; ++h) tma_load_2d(dst + h * cfg::kWBytes, map_w[h], kb * cfg::BK, n0, full_bar(s));
+      };
+      auto load_a = [&](int kb, int s) {
+        const uint32_t dst = base + s * cfg::kStageBytes;
+#pragma unroll
+        for (int h = 0; h < cfg::kParts; ++h) tma_load_2d(dst + h * cfg::kABytes, map_a[h], kb * cfg::BK, m0, full_bar(s));
+      };
+      const int first = min(kb1 - kb0, S);
+      if (weights_ready) {
+        for (int i = 0; i < first; ++i) load_w(kb0 + i, i);
+        pdl_wait();
+        for (int i = 0; i < first; ++i) load_a(kb0 + i, i);
+      } else {
+        pdl_wait();
+        for (int i = 0; i < first; ++i) {
+          load_w(kb0 + i, i);
+          load_a(kb0 + i, i);
+        }
+      }
+      int issued = first;
+      // a tile beyond the valid rows stops here (the first tile needs no look: it has rows unless M is 0)
+      const bool live = blockIdx.z == 0 || valid_rows() > 0;
+      if (live) {
+        for (; issued < kb1 - kb0; ++issued) {
+          const int s = issued % S;
+          if (!mbar_wait(empty_bar(s), static_cast<uint32_t>((issued / S - 1) & 1), abort_flag)) {
+            fail(kSiteProducer);
+            break;
+          }
+          load_w(kb0 + issued, s);
+          load_a(kb0 + issued, s);
+        }
+      }
+      // copies in flight must land before the CTA's shared memory goes away
+      for (int i = max(0, issued - S); i < issued; ++i)
+        if (!mbar_wait(full_bar(i % S), static_cast<uint32_t>((i / S) & 1), abort_flag) && *abort_flag == 0)
+          fail(kSiteDrain);
+    } else {
+      pdl_wait();
+      if (lane == 0) report_timeout(status_word, kKernelGemmTc, 16 + kSiteAlign);
+    }
+    __syncwarp();
+    if (splits > 1) {
+      cluster_wait();
+      cluster_arrive();
+      cluster_wait();
+    }
+  } else if (warp == 1) {
+    // ------------------------- MMA issuer -------------------------
+    pdl_wait();
+    if (lane == 0 && aligned && (blockIdx.z == 0 || valid_rows() > 0)) {
+      constexpr uint32_t idesc = make_idesc_f16_f32acc(BM, BN) | (kTf32 ? (2u << 7) | (2u << 10) : 0u);
+      bool ok = true;
+      for (int i = 0; i < kb1 - kb0; ++i) {
+        const int s = i % S;
+        if (!mbar_wait(full_bar(s), static_cast<uint32_t>((i / S) & 1), abort_flag)) {
+          fail(kSiteMma);
+          ok = false;
+          break;
+        }
+        tc_fence_after();
+        const uint32_t a = base + s * cfg::kStageBytes, w = a + cfg::kParts * cfg::kABytes;
+        const uint32_t d = tmem_base + (i / cfg::kUnitKb) * BN;
+        const bool fresh = i % cfg::kUnitKb == 0;
+        const uint64_t ad = make_kmajor_sw128_desc(a), wd = make_kmajor_sw128_desc(w);
+        if constexpr (kTf32) {
+          const uint64_t ad2 = make_kmajor_sw128_desc(a + cfg::kABytes), wd2 = make_kmajor_sw128_desc(w + cfg::kWBytes);
+#pragma unroll
+          for (int k = 0; k < 4; ++k) umma_tf32_ss(d, ad + 2u * k, wd + 2u * k, idesc, (!fresh || k > 0) ? 1u : 0u);
+#pragma unroll
+          for (int k = 0; k < 4; ++k) umma_tf32_ss(d, ad + 2u * k, wd2 + 2u * k, idesc, 1u);
+#pragma unroll
+          for (int k = 0; k < 4; ++k) umma_tf32_ss(d, ad2 + 2u * k, wd + 2u * k, idesc, 1u);
+        } else {
+#pragma unroll
+          for (int k = 0; k < 4; ++k) umma_f16_ss(d, ad + 2u * k, wd + 2u * k, idesc, (!fresh || k > 0) ? 1u : 0u);
+        }
+        umma_commit(empty_bar(s));
+      }
+      if (ok) umma_commit(acc_bar);
+      umma_commit(drain_bar);
+      if (!mbar_wait(drain_bar, 0u, abort_flag) && *abort_flag == 0) fail(kSiteMmaDrain);
+    }
+    __syncwarp();
+    if (splits > 1) {
+      cluster_wait();
+      cluster_arrive();
+      cluster_wait();
+    }
+  } else {
+    // ------------------------- partial sums, reduction, epilogue -------------------------
+    pdl_wait();
+    const int rows = valid_rows();
+    const bool live = rows > 0 && aligned;
+    const int quad = warp & 3;
+    const int t = threadIdx.x - 64;      // 0..127
+    const int piece = t & 7;             // this thread's eight columns
+    const int col = n0 + piece * 8;
+    const int items = 8 / splits;        // rows of this thread: rank + splits * ((t >> 3) + 16 * j)
+    auto row_of = [&](int j) { return rank + splits * ((t >> 3) + 16 * j); };
+    T* C = static_cast<T*>(c_ptr);
+    const T* bias = static_cast<const T*>(bias_ptr);
+    const T* residual = static_cast<const T*>(res_ptr);
+
+    // what the epilogue needs beside the sums is requested before the accumulator is waited for
+    float fb[8], fg[8], fe[8];
+    Vec16 res[8];
+    float2 st[8][2];
+#pragma unroll
+    for (int e = 0; e < 8; ++e) fb[e] = 0.f, fg[e] = 1.f, fe[e] = 0.f;
+    if (live) {
+      if (EPI != kEpiNone) load8(bias + col, fb);
+      if constexpr (EPI == kEpiNormResidual) {
+        if (ln.gamma != nullptr) {
+          load8(ln.gamma + col, fg);
+          load8(ln.beta + col, fe);
+        }
+      }
+      if constexpr (kNormIn) load8(ln.csum + col, fg);
+#pragma unroll
+      for (int j = 0; j < 8; ++j)
+        if (j < items && row_of(j) < rows) {
+          if constexpr (kResidual) res[j] = ld_global_nc_v4(residual + static_cast<size_t>(m0 + row_of(j)) * N + col);
+          if constexpr (is_deferred_norm(EPI)) {
+            st[j][0] = st[j][1] = make_float2(0.f, 0.f);
+            if (ln.stats_in != nullptr) {
+              const float2* sp = reinterpret_cast<const float2*>(ln.stats_in) + static_cast<size_t>(m0 + row_of(j)) * ln.stat_slots;
+              if (piece < ln.stat_slots) st[j][0] = sp[piece];
+              if (piece + 8 < ln.stat_slots) st[j][1] = sp[piece + 8];
+            }
+          }
+        }
+    }
+
+    bool got = live;
+    if (live) {
+      got = __all_sync(0xffffffffu, mbar_wait(acc_bar, 0u, abort_flag));
+      if (!got && lane == 0) fail(kSiteEpilogue);
+    }
+    if (splits > 1) cluster_wait();  // (the first arrival: every CTA has started)
+    if (got && quad * 32 < rows) {
+      tc_fence_after();
+      const uint32_t t_row = tmem_base + (static_cast<uint32_t>(quad * 32) << 16);
+      const int r = quad * 32 + lane;
+      const int slot = r / splits;
+      const uint32_t dst0 = recv + ((rank * (BM / splits) + slot) * BN) * 4;
+      const uint32_t dst = splits > 1 ? mapa_shared(dst0, r % splits) : dst0;
+#pragma unroll
+      for (int hcol = 0; hcol < 2; ++hcol) {
+        float sum[32];
+#pragma unroll
+        for (int e = 0; e < 32; ++e) sum[e] = 0.f;
+        for (int u = 0; u < units; ++u) {
+          uint32_t v[32];
+          tmem_ld_32x32b_x32(t_row + u * BN + hcol * 32, v);
+          tmem_ld_wait();
+#pragma unroll
+          for (int e = 0; e < 32; ++e) sum[e] += __uint_as_float(v[e]);
+        }
+        if (r < rows) {
+#pragma unroll
+          for (int g = 0; g < 8; ++g) {
+            // 16-byte groups swizzled by the row's slot: the readers' and the writers' banks are spread
+            const uint32_t at = dst + (((hcol * 8 + g) ^ (slot & 15)) << 4);
+            if (splits > 1) st_cluster_v4(at, sum[4 * g], sum[4 * g + 1], sum[4 * g + 2], sum[4 * g + 3]);
+            else asm volatile("st.shared.v4.f32 [%0], {%1,%2,%3,%4};" ::"r"(at), "f"(sum[4 * g]), "f"(sum[4 * g + 1]),
+                              "f"(sum[4 * g + 2]), "f"(sum[4 * g + 3]) : "memory");
+          }
+        }
+      }
+      tc_fence_before();
+    }
+    __syncwarp();
+    if (splits > 1) {
+      cluster_arrive();
+      cluster_wait();
+    } else {
+      asm volatile("bar.sync 1, %0;" ::"n"(kEpThreads) : "memory");
+    }
+    if (live && *abort_flag == 0) {
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        if (j >= items) break;           // uniform
+        const int r = row_of(j);
+        const int slot = (t >> 3) + 16 * j;
+        const bool mine = r < rows;      // uniform in the eight lanes of a row
+        float f[8];
+#pragma unroll
+        for (int e = 0; e < 8; ++e) f[e] = 0.f;
+        if (mine) {
+          for (int src = 0; src < splits; ++src) {
+            const uint32_t rowp = recv + ((src * (BM / splits) + slot) * BN) * 4;
+            const float4 p0 = ld_shared_f4(rowp + (((2 * piece) ^ (slot & 15)) << 4));
+            const float4 p1 = ld_shared_f4(rowp + (((2 * piece + 1) ^ (slot & 15)) << 4));
+            f[0] += p0.x, f[1] += p0.y, f[2] += p0.z, f[3] += p0.w;
+            f[4] += p1.x, f[5] += p1.y, f[6] += p1.z, f[7] += p1.w;
+          }
+        }
+        float mu = 0.f, rstd = 1.f;
+        if constexpr (is_deferred_norm(EPI)) {
+          float a = mine ? st[j][0].x + st[j][1].x : 0.f, b = mine ? st[j][0].y + st[j][1].y : 0.f;
+#pragma unroll
+          for (int o = 1; o < 8; o <<= 1) {
+            a += __shfl_xor_sync(0xffffffffu, a, o);
+            b += __shfl_xor_sync(0xffffffffu, b, o);
+          }
+          if (ln.stats_in != nullptr) {
+            const float inv = 1.0f / static_cast<float>(ln.stat_slots * 64);
+            mu = a * inv;
+            rstd = rsqrtf(fmaxf(b * inv - mu * mu, 0.f) + ln.eps);
+          }
+        }
+        const size_t at = static_cast<size_t>(m0 + r) * N + col;
+        if constexpr (kTf32) {
+#pragma unroll
+          for (int e = 0; e < 8; ++e) {
+            if (EPI != kEpiNone) f[e] += fb[e];
+            if (EPI == kEpiBiasGelu) f[e] = gelu_tanh(f[e]);
+            if (EPI == kEpiBiasTanh) f[e] = tanhf(f[e]);
+          }
+          if (mine) {
+            if (c_lo != nullptr) {
+              float lo[8];
+#pragma unroll
+              for (int e = 0; e < 8; ++e) {
+                const float hi = rn_tf32(f[e]);
+                lo[e] = f[e] - hi;
+                f[e] = hi;
+              }
+              st_global_v4(c_lo + at, VecTraits<float>::pack(lo));
+              st_global_v4(c_lo + at + 4, VecTraits<float>::pack(lo + 4));
+            }
+            st_global_v4(C + at, VecTraits<float>::pack(f));
+            st_global_v4(C + at + 4, VecTraits<float>::pack(f + 4));
+          }
+        } else {
+          if constexpr (kNormIn) {
+            // rstd * (acc - mu * csum[n]) + bias[n]
+#pragma unroll
+            for (int e = 0; e < 8; ++e) f[e] = fmaf(rstd, fmaf(-mu, fg[e], f[e]), fb[e]);
+          } else if constexpr (EPI == kEpiNormResidual) {
+            // (res - mu) * rstd in fp32: see epilogue_warp_tile in gemm_tcgen05.cu
+            float fr[8];
+            VecTraits<__half>::unpack(res[j], fr);
+            const float nmr = -mu * rstd;
+#pragma unroll
+            for (int e = 0; e < 8; ++e) f[e] += fb[e] + fmaf(fmaf(fr[e], rstd, nmr), fg[e], fe[e]);
+          } else if constexpr (EPI != kEpiNone) {
+#pragma unroll
+            for (int e = 0; e < 8; ++e) f[e] += fb[e];
+          }
+          if constexpr (EPI == kEpiBiasResidual) {
+            float fr[8];
+            VecTraits<__half>::unpack(res[j], fr);
+#pragma unroll
+            for (int e = 0; e < 8; ++e) f[e] += fr[e];
+          }
+          if constexpr (EPI == kEpiBiasTanh) {
+#pragma unroll
+            for (int e = 0; e < 8; ++e) f[e] = tanhf(f[e]);
+          }
+          Vec16 o = VecTraits<__half>::pack(f);
+          if constexpr (EPI == kEpiBiasGelu || EPI == kEpiNormInGelu) {
+            o.x = gelu_tanh_half2(o.x);
+            o.y = gelu_tanh_half2(o.y);
+            o.z = gelu_tanh_half2(o.z);
+            o.w = gelu_tanh_half2(o.w);
+          }
+          if (mine) st_global_v4(C + at, o);
+          if constexpr (EPI == kEpiNormResidual) {
+            // statistics of the row's 64-column piece as stored
+            float y[8], a = 0.f, b = 0.f;
+            VecTraits<__half>::unpack(o, y);
+#pragma unroll
+            for (int e = 0; e < 8; ++e) {
+              a += y[e];
+              b = fmaf(y[e], y[e], b);
+            }
+#pragma unroll
+            for (int o2 = 1; o2 < 8; o2 <<= 1) {
+              a += __shfl_xor_sync(0xffffffffu, a, o2);
+              b += __shfl_xor_sync(0xffffffffu, b, o2);
+            }
+            if (mine && piece == 0)
+              reinterpret_cast<float2*>(ln.stats_out)[static_cast<size_t>(m0 + r) * (N / 64) + blockIdx.y] = make_float2(a, b);
+          }
+        }
+      }
+    }
+  }
+
+  tc_fence_before();
+  __syncthreads();
+  if (warp == 1) {
+    __syncwarp();
+    tc_fence_after();
+    tmem_dealloc(tmem_base, cfg::kTmemCols);
+  }
+}
+
+template <bool kTf32, int EPI>
+cudaError_t launch_split(const Maps& maps, const SplitGemm& g, int splits, cudaStream_t stream) {
+  using cfg = Cfg<kTf32>;
+  static PerDeviceOnce once;  // function attributes are per device
+  const cudaError_t once_err = once.run([] {
+    return cudaFuncSetAttribute(gemm_split_kernel<kTf32, EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                cfg::kSmemBytes);
+  });
+  if (once_err != cudaSuccess) return once_err;
+  cudaLaunchConfig_t lc = {};
+  lc.gridDim = dim3(splits, g.n / BN, (g.max_m + BM - 1) / BM);
+  lc.blockDim = dim3(kThreads);
+  lc.dynamicSmemBytes = cfg::kSmemBytes;
+  lc.stream = stream;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = splits;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
+  lc.attrs = attr;
+  lc.numAttrs = pdl_enabled() ? 2 : 1;
+  return cudaLaunchKernelEx(&lc, gemm_split_kernel<kTf32, EPI>, maps, g.c, g.c_lo, g.bias, g.residual, g.m_ptr,
+                            g.max_m, g.n, (g.k + cfg::BK - 1) / cfg::BK, g.weights_ready ? 1 : 0, g.status_word, g.ln);
+}
+
+bool encode_split(CUtensorMap* map, bool tf32, const void* base, int rows, int k, int box_rows, TensorMapCache* cache) {
+  return tf32 ? encode_2d_f32_sw128(map, base, rows, k, box_rows, cache)
+              : encode_2d_fp16_sw128(map, base, rows, k, k, box_rows, 64, cache);
+}
+
+}  // namespace
+
+// Where a cluster's split pays, from the capacity in rows (the valid rows are only known on the device).
+// One B200, us per launch, rows = 0.6 * capacity, 1 / 2 / 4 / 8 CTAs per tile against the persistent kernel:
+//   fp16, N x K     capacity 64                      512                            2048
+//   768 x 768       6.9  5.1  4.1  4.4 (7.9)         8.2  6.8  7.4 10.2 ( 8.5)      8.7  9.3  17  34 ( 8.7)
+//   2304 x 768      7.2  5.3  5.4  9.1 (8.2)         8.5  7.9 14.4 26.8 ( 9.1)     16.8 25.1  50  98 (10.1)
+//   768 x 3072     17.3 10.3  6.8  5.6 (18.6)       19.5 12.4 10.2 13.1 (19.5)     20.2 14.3  24  42 (20.1)
+//   fp32, N x K
+//   2304 x 768     17.9 11.0 14.7 17.9 (17.4)       19.6 23.2 32.7 57.9 (17.7)
+//   768 x 3072     55.1 30.3 17.1 11.1 (55.1)       54.7 31.8 34.3 34.4 (54.6)
+// So: as many CTAs per tile as still run at once (two fp16 CTAs per SM, one fp32), each with enough of K to
+// hide its load latency: six 64-wide or twelve 32-wide steps, or three where the grid is small enough (two
+// thirds of the SMs) not to share L2 bandwidth.  From six row tiles on a third more CTAs than run at once is
+// taken, if their share of K is long: a batch has padding, and the tiles it leaves empty cost next to nothing.
+int gemm_split_count(int max_m, int n, int k, bool tf32) {
+  if (n % BN != 0 || max_m <= 0) return 0;
+  const int num_kb = (k + (tf32 ? 31 : 63)) / (tf32 ? 32 : 64);
+  const long long m_tiles = (max_m + BM - 1) / BM, tiles = m_tiles * (n / BN);
+  const long long sms = sm_count(), at_once = sms * (tf32 ? 1 : 2);
+  for (int splits = kMaxSplits; splits >= 1; splits >>= 1) {
+    const int share = num_kb / splits;
+    const long long ctas = tiles * splits;
+    if (share < 1 || (tf32 && (num_kb + splits - 1) / splits > Cfg<true>::kBlocks * Cfg<true>::kUnitKb)) continue;
+    if (splits == 1) return tf32 || ctas > at_once ? 0 : 1;  // fp32: no better than the 128 x 128 tiles
+    if (share < 3 || (share < (tf32 ? 12 : 6) && 3 * ctas > 2 * sms)) continue;
+    if (ctas <= at_once || (m_tiles >= 6 && share >= 12 && 3 * ctas <= 4 * at_once)) return splits;
+  }
+  return 0;
+}
+
+cudaError_t launch_gemm_split(const SplitGemm& g, int epilogue, int splits, TensorMapCache* maps, cudaStream_t stream) {
+  const bool tf32 = g.a_lo != nullptr;
+  Maps m;
+  if (!encode_split(&m.a, tf32, g.a, g.max_m, g.k, BM, maps) || !encode_split(&m.w, tf32, g.w, g.n, g.k, BN, maps))
+    return cudaErrorInvalidValue;
+  m.a_lo = m.a, m.w_lo = m.w;
+  if (tf32 && (!encode_split(&m.a_lo, true, g.a_lo, g.max_m, g.k, BM, maps) ||
+               !encode_split(&m.w_lo, true, g.w_lo, g.n, g.k, BN, maps)))
+    return cudaErrorInvalidValue;
+#define ETB_CASE(TF, E) \
+  case E:               \
+    return launch_split<TF, E>(m, g, splits, stream)
+  if (tf32) {
+    switch (epilogue) {
+      ETB_CASE(true, kEpiNone);
+      ETB_CASE(true, kEpiBias);
+      ETB_CASE(true, kEpiBiasGelu);
+      ETB_CASE(true, kEpiBiasTanh);
+      default:
+        return cudaErrorInvalidValue;
+    }
+  }
+  switch (epilogue) {
+    ETB_CASE(false, kEpiNone);
+    ETB_CASE(false, kEpiBias);
+    ETB_CASE(false, kEpiBiasGelu);
+    ETB_CASE(false, kEpiBiasTanh);
+    ETB_CASE(false, kEpiBiasResidual);
+    ETB_CASE(false, kEpiNormIn);
+    ETB_CASE(false, kEpiNormInGelu);
+    ETB_CASE(false, kEpiNormResidual);
+    default:
+      return cudaErrorInvalidValue;
+  }
+#undef ETB_CASE
+}
+
+}  // namespace etb

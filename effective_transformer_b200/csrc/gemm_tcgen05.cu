@@ -1320,7 +1320,7 @@ bool encode_2d_fp16_sw128(CUtensorMap* map, const void* base, uint64_t rows, uin
 cudaError_t launch_gemm_tcgen05(const __half* a, const __half* w_packed, const __half* bias,
                                 __half* c, const int* m_ptr, int max_m, int n, int k, int epilogue,
                                 int* status_word, cudaStream_t stream, bool reverse_m, const __half* residual,
-                                TensorMapCache* maps, const GemmLayerNorm* ln) {
+                                TensorMapCache* maps, const GemmLayerNorm* ln, bool weights_ready) {
   if (max_m <= 0) return cudaSuccess;
   if (n <= 0 || k <= 0 || (n % 128) != 0 || (k % 8) != 0) return cudaErrorInvalidValue;
   if ((reinterpret_cast<uintptr_t>(a) & 15u) || (reinterpret_cast<uintptr_t>(w_packed) & 15u) ||
@@ -1358,6 +1358,15 @@ cudaError_t launch_gemm_tcgen05(const __half* a, const __half* w_packed, const _
       if (ln->csum == nullptr || (reinterpret_cast<uintptr_t>(ln->csum) & 15u)) return cudaErrorInvalidValue;
     }
     lnp = *ln;
+  }
+  if (const int splits = has_ln(epilogue) ? 0 : gemm_split_count(max_m, n, k, false)) {
+    SplitGemm g;
+    g.a = a, g.w = w_packed, g.bias = bias, g.residual = residual, g.c = c;
+    g.m_ptr = m_ptr, g.max_m = max_m, g.n = n, g.k = k;
+    g.weights_ready = weights_ready;
+    g.status_word = status_word;
+    g.ln = lnp;
+    return launch_gemm_split(g, epilogue, splits, maps, stream);
   }
   const int bn = (n % 256 == 0) ? 256 : 128;
   const bool pair = bn == 256;

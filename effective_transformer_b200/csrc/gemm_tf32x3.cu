@@ -727,28 +727,6 @@ gemm_tf32x3_pair_kernel(const __grid_constant__ CUtensorMap tmap_a_hi, const __g
   }
 }
 
-bool encode_2d_f32_sw128(CUtensorMap* map, const void* base, uint64_t rows, uint64_t cols, uint32_t box_rows,
-                         TensorMapCache* cache) {
-  if (cache != nullptr) {
-    if (const CUtensorMap* hit = cache->find(4, base, rows, cols, cols, box_rows, BK)) {
-      *map = *hit;
-      return true;
-    }
-  }
-  EncodeTiledFn fn = get_encode_tiled();
-  if (fn == nullptr) return false;
-  const cuuint64_t dims[2] = {cols, rows};
-  const cuuint64_t strides[1] = {cols * 4};
-  const cuuint32_t box[2] = {static_cast<cuuint32_t>(BK), box_rows};
-  const cuuint32_t elem_strides[2] = {1, 1};
-  const CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, const_cast<void*>(base), dims, strides, box,
-                        elem_strides, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
-                        CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  if (r != CUDA_SUCCESS) return false;
-  if (cache != nullptr) cache->insert(4, base, rows, cols, cols, box_rows, BK, *map);
-  return true;
-}
-
 template <int EPI>
 cudaError_t launch_epi(const CUtensorMap& tah, const CUtensorMap& tal, const CUtensorMap& twh, const CUtensorMap& twl,
                        const float* bias, float* c, float* c_lo, const int* m_ptr, int max_m, int n, int k,
@@ -791,6 +769,28 @@ cudaError_t launch_pair_epi(const CUtensorMap& tah, const CUtensorMap& tal, cons
 
 }  // namespace
 
+bool encode_2d_f32_sw128(CUtensorMap* map, const void* base, uint64_t rows, uint64_t cols, uint32_t box_rows,
+                         TensorMapCache* cache) {
+  if (cache != nullptr) {
+    if (const CUtensorMap* hit = cache->find(4, base, rows, cols, cols, box_rows, BK)) {
+      *map = *hit;
+      return true;
+    }
+  }
+  EncodeTiledFn fn = get_encode_tiled();
+  if (fn == nullptr) return false;
+  const cuuint64_t dims[2] = {cols, rows};
+  const cuuint64_t strides[1] = {cols * 4};
+  const cuuint32_t box[2] = {static_cast<cuuint32_t>(BK), box_rows};
+  const cuuint32_t elem_strides[2] = {1, 1};
+  const CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, const_cast<void*>(base), dims, strides, box,
+                        elem_strides, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
+                        CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  if (r != CUDA_SUCCESS) return false;
+  if (cache != nullptr) cache->insert(4, base, rows, cols, cols, box_rows, BK, *map);
+  return true;
+}
+
 cudaError_t launch_split_tf32(const float* x, float* hi, float* lo, const int* rows_ptr, int max_rows, int cols,
                               cudaStream_t stream) {
   if (max_rows <= 0 || cols <= 0) return cudaSuccess;
@@ -806,7 +806,7 @@ cudaError_t launch_split_tf32(const float* x, float* hi, float* lo, const int* r
 cudaError_t launch_gemm_tf32x3(const float* a_hi, const float* a_lo, const float* w_hi, const float* w_lo,
                                const float* bias, float* c, const int* m_ptr, int max_m, int n, int k,
                                int epilogue, int* status_word, cudaStream_t stream, bool reverse_m, float* c_lo,
-                               TensorMapCache* maps) {
+                               TensorMapCache* maps, bool weights_ready) {
   if (max_m <= 0) return cudaSuccess;
   if (n <= 0 || k <= 0 || (n % 128) != 0 || (k % BK) != 0) return cudaErrorInvalidValue;
   for (const void* p : {static_cast<const void*>(a_hi), static_cast<const void*>(a_lo),
@@ -816,6 +816,14 @@ cudaError_t launch_gemm_tf32x3(const float* a_hi, const float* a_lo, const float
   if (bias != nullptr && (reinterpret_cast<uintptr_t>(bias) & 15u)) return cudaErrorMisalignedAddress;
   if (c_lo != nullptr && (reinterpret_cast<uintptr_t>(c_lo) & 15u)) return cudaErrorMisalignedAddress;
   if (epilogue != kEpiNone && bias == nullptr) return cudaErrorInvalidValue;
+  if (const int splits = gemm_split_count(max_m, n, k, true)) {
+    SplitGemm g;
+    g.a = a_hi, g.a_lo = a_lo, g.w = w_hi, g.w_lo = w_lo, g.bias = bias, g.c = c, g.c_lo = c_lo;
+    g.m_ptr = m_ptr, g.max_m = max_m, g.n = n, g.k = k;
+    g.weights_ready = weights_ready;
+    g.status_word = status_word;
+    return launch_gemm_split(g, epilogue, splits, maps, stream);
+  }
   CUtensorMap tah, tal, twh, twl;
   if (!encode_2d_f32_sw128(&tah, a_hi, static_cast<uint64_t>(max_m), static_cast<uint64_t>(k), BM, maps) ||
       !encode_2d_f32_sw128(&tal, a_lo, static_cast<uint64_t>(max_m), static_cast<uint64_t>(k), BM, maps) ||

@@ -298,5 +298,8 @@ class TensorMapCache {
 bool encode_2d_fp16_sw128(CUtensorMap* map, const void* base, uint64_t rows, uint64_t cols,
                           uint64_t row_stride_elems, uint32_t box_rows, uint32_t box_cols,
                           TensorMapCache* cache = nullptr);
+// fp32 row-major [rows, cols] tensor, box [box_rows, 32], 128-byte swizzle.
+bool encode_2d_f32_sw128(CUtensorMap* map, const void* base, uint64_t rows, uint64_t cols, uint32_t box_rows,
+                         TensorMapCache* cache);
 
 }  // namespace etb

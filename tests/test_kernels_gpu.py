@@ -432,6 +432,35 @@ def test_gemm_fp32_on_tensor_cores_keeps_fp32_accuracy(m, cap, n, k, epi):
         assert float((one_term - plain).abs().max()) > 20 * float((c[:m].double() - ref).abs().max()) or k < 128
 
 
+# Small batches, whose projections split a tile's K range over a cluster (1, 2, 4 and 8 CTAs per tile):
+# fewer rows than CTAs, a row tile's edges, a last tile with one row, a row tile the batch leaves empty, K that
+# does not divide evenly (or at all: fp16 K of 8), N of an odd number of 64-column tiles per 128.
+SPLIT_SHAPES = [(3, 64, 768, 3072), (127, 128, 768, 768), (128, 128, 2304, 768), (129, 256, 768, 3072),
+                (40, 256, 3072, 768), (385, 700, 768, 3072), (500, 512, 384, 1600), (600, 640, 1024, 4096),
+                (513, 768, 3072, 768)]
+
+
+@pytest.mark.parametrize("m,cap,n,k", SPLIT_SHAPES + [(77, 90, 256, 1000), (5, 8, 128, 72)])
+@pytest.mark.parametrize("epi", [0, 1, 2])
+def test_gemm_tcgen05_k_range_split_over_a_cluster(m, cap, n, k, epi):
+    _gemm_case(torch.float16, m, cap, n, k, epi, use_simt=False)
+
+
+@pytest.mark.parametrize("m,cap,n,k", SPLIT_SHAPES)
+@pytest.mark.parametrize("epi", [0, 1, 2, 3])
+def test_gemm_fp32_k_range_split_over_a_cluster(m, cap, n, k, epi):
+    test_gemm_fp32_on_tensor_cores_keeps_fp32_accuracy(m, cap, n, k, epi)
+
+
+@pytest.mark.parametrize("m,cap,n,k", [s for s in SPLIT_SHAPES if s[2] % 256 == 0])
+def test_gemm_k_range_split_with_the_layer_epilogues(m, cap, n, k):
+    _gemm_fused_case(m, cap, n, k, 4)
+    if n <= 1024:
+        _deferred_producer_case(m, cap, n, k, True)
+    if k <= 1024:
+        _deferred_consumer_case(m, cap, n, k, True, True)
+
+
 # ---- epilogues that take the layer's residual: bias + residual, and the LayerNorm inside the GEMM -------
 def _gemm_fused_case(m, cap, n, k, epi, seed=0, counters_check=True):
     """et_gemm_fused against the float64 oracle: C = A W + bias + residual (4), and its LayerNorm
