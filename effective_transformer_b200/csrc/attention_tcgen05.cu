@@ -197,7 +197,47 @@ struct MaskArgs {
   const int* batch_idx;
   const int* word_idx;
   int seq;
+  const uint32_t* bits;  // rows of mask_bits_kernel (one look per batch), null: every item reads the mask itself
 };
+
+// What a query row of the packed tensor may attend to, worked out once per batch: kMaskBitsStride words per
+// token, [0,4) a bit per key of its own sequence (key i = token seq_lo + i), [4] the number of padded key
+// positions it may attend to, as a float.  A warp per token, lanes over the row's keys, so that a mask row is
+// read in whole lines; in the attention kernel a thread reads its row alone, twice, key by key, and again for
+// every head of every layer.
+constexpr int kMaskBitsStride = 8;
+__global__ void __launch_bounds__(256)
+mask_bits_kernel(const __half* __restrict__ attr_mask, const int* __restrict__ batch_idx,
+                 const int* __restrict__ word_idx, const int* __restrict__ cu_seqlens, const int* __restrict__ t_ptr,
+                 int max_tokens, int seq, uint32_t* __restrict__ out) {
+  pdl_wait();
+  pdl_trigger();
+  const int lane = threadIdx.x & 31;
+  const int tokens = min(max(*t_ptr, 0), max_tokens);
+  for (int t = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; t < tokens; t += (gridDim.x * blockDim.x) >> 5) {
+    const int b = batch_idx[t];
+    const int lo = max(cu_seqlens[b], 0);
+    const int len = min(min(cu_seqlens[b + 1], max_tokens) - lo, kTileRows);
+    const __half* mrow = attr_mask + (static_cast<size_t>(b) * seq + word_idx[t]) * seq;
+    int total = 0;  // allowed key positions, valid or padded
+    for (int j0 = 0; j0 < seq; j0 += 32) {
+      const int j = j0 + lane;
+      total += __popc(__ballot_sync(0xffffffffu, j < seq && __half2float(mrow[j]) > 0.5f));
+    }
+    int allowed = 0;
+    uint32_t mine = 0u;
+#pragma unroll
+    for (int w = 0; w < 4; ++w) {
+      const int i = w * 32 + lane;
+      const bool a = i < len && (total == 0 || __half2float(mrow[word_idx[lo + i]]) > 0.5f);
+      const uint32_t word = __ballot_sync(0xffffffffu, a);
+      allowed += __popc(word);
+      if (lane == w) mine = word;
+    }
+    if (lane == 4) mine = __float_as_uint(static_cast<float>(total == 0 ? seq - len : total - allowed));
+    if (lane < 5) out[static_cast<size_t>(t) * kMaskBitsStride + lane] = mine;
+  }
+}
 
 template <bool kMask>
 __global__ void __launch_bounds__(kThreads, kCtasPerSm)
@@ -337,7 +377,20 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_q, const __gri
     uint32_t allow[4] = {0u, 0u, 0u, 0u};
     float n_pad = 0.f;
     if constexpr (kMask) {
-      if (r < n && hi > lo) {
+      if (r < n && hi > lo && ma.bits != nullptr) {
+        const uint32_t* bp = ma.bits + static_cast<size_t>(t0 + r) * kMaskBitsStride;
+        const uint4 bw = *reinterpret_cast<const uint4*>(bp);
+        n_pad = __uint_as_float(bp[4]);
+        // key i of the sequence is tile column lo + i: the 128 bits move up by lo
+        allow[0] = bw.x, allow[1] = bw.y, allow[2] = bw.z, allow[3] = bw.w;
+        if (lo & 64) allow[3] = allow[1], allow[2] = allow[0], allow[1] = 0u, allow[0] = 0u;
+        if (lo & 32) allow[3] = allow[2], allow[2] = allow[1], allow[1] = allow[0], allow[0] = 0u;
+        const uint32_t sh = static_cast<uint32_t>(lo & 31);
+        allow[3] = __funnelshift_l(allow[2], allow[3], sh);
+        allow[2] = __funnelshift_l(allow[1], allow[2], sh);
+        allow[1] = __funnelshift_l(allow[0], allow[1], sh);
+        allow[0] <<= sh;
+      } else if (r < n && hi > lo) {
         const int token = t0 + r;
         const __half* mrow = ma.attr_mask +
             (static_cast<size_t>(ma.batch_idx[token]) * ma.seq + ma.word_idx[token]) * ma.seq;
@@ -808,11 +861,24 @@ cudaError_t launch_attention_plan(const int* cu_seqlens, int batch, int max_toke
   return cudaGetLastError();
 }
 
+size_t attention_mask_bits_words(size_t max_tokens) { return max_tokens * kMaskBitsStride; }
+
+cudaError_t launch_attention_mask_bits(const __half* attr_mask, const int* batch_idx, const int* word_idx,
+                                       const int* cu_seqlens, const int* t_ptr, int max_tokens, int seq,
+                                       uint32_t* bits, cudaStream_t stream) {
+  if (max_tokens <= 0) return cudaSuccess;
+  if (seq <= 0 || seq > kTileRows) return cudaErrorInvalidValue;
+  const int ctas = min((max_tokens + 7) / 8, sm_count() * 8);
+  return launch_pdl(mask_bits_kernel, dim3(ctas), dim3(256), 0, stream, attr_mask, batch_idx, word_idx, cu_seqlens,
+                    t_ptr, max_tokens, seq, bits);
+}
+
 cudaError_t launch_attention_tcgen05(const __half* q, const __half* k, const __half* v,
                                      long long token_stride, long long head_stride, __half* ctx,
                                      const int* plan, int batch, int max_tokens, int heads, int d,
                                      int* status_word, cudaStream_t stream, bool reverse, TensorMapCache* maps,
-                                     const __half* attr_mask, const int* batch_idx, const int* word_idx, int seq) {
+                                     const __half* attr_mask, const int* batch_idx, const int* word_idx, int seq,
+                                     const uint32_t* mask_bits) {
   if (batch <= 0 || heads <= 0 || max_tokens <= 0) return cudaSuccess;
   if (d != kD || token_stride < kD || (token_stride % 8) != 0 || (head_stride % 8) != 0 || head_stride < 0)
     return cudaErrorInvalidValue;
@@ -840,7 +906,7 @@ cudaError_t launch_attention_tcgen05(const __half* q, const __half* k, const __h
   const bool masked = attr_mask != nullptr;
   if (masked && (batch_idx == nullptr || word_idx == nullptr || seq <= 0 || seq > kTileRows))
     return cudaErrorInvalidValue;
-  const MaskArgs ma{attr_mask, batch_idx, word_idx, seq};
+  const MaskArgs ma{attr_mask, batch_idx, word_idx, seq, mask_bits};
   const float scale_log2e = (1.0f / sqrtf(static_cast<float>(d))) * 1.4426950408889634f;
   // every tile holds at least one sequence, so batch * heads bounds the item count
   long long grid = static_cast<long long>(sm_count()) * kCtasPerSm;

@@ -384,7 +384,13 @@ cudaError_t launch_attention_tcgen05(const __half* q, const __half* k, const __h
                                      const int* plan, int batch, int max_tokens, int heads, int d,
                                      int* status_word, cudaStream_t stream, bool reverse = false,
                                      TensorMapCache* maps = nullptr, const __half* attr_mask = nullptr,
-                                     const int* batch_idx = nullptr, const int* word_idx = nullptr, int seq = 0);
+                                     const int* batch_idx = nullptr, const int* word_idx = nullptr, int seq = 0,
+                                     const uint32_t* mask_bits = nullptr);
+// The general mask as bits per token, once per batch, for the launches of its layers (mask_bits above).
+size_t attention_mask_bits_words(size_t max_tokens);
+cudaError_t launch_attention_mask_bits(const __half* attr_mask, const int* batch_idx, const int* word_idx,
+                                       const int* cu_seqlens, const int* t_ptr, int max_tokens, int seq,
+                                       uint32_t* bits, cudaStream_t stream);
 // fp32 GEMM on the tensor cores by the three-product tf32 split (gemm_tf32x3.cu):
 // x = hi + lo with hi = rn_tf32(x); hi/lo may alias x.  rows_ptr null = max_rows.
 cudaError_t launch_split_tf32(const float* x, float* hi, float* lo, const int* rows_ptr, int max_rows, int cols,

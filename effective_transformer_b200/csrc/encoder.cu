@@ -103,6 +103,7 @@ struct Workspace {
   int* lens_scratch = nullptr;
   int* attn_plan = nullptr;   // tile plan of the tcgen05 attention (made once per batch)
   int* pos_row = nullptr;     // [B*S] position -> packed row (general-mask attention)
+  uint32_t* mask_bits = nullptr;  // a general mask as bits per token (attention on packed tiles)
   float* a_hi = nullptr;      // fp32 handles: [cap, H] tf32 halves of a projection's input
   float* a_lo = nullptr;
   float* ffn_lo = nullptr;    // fp32 handles: [cap, F] remainder of the GELU output (its tf32 half is in ffn)
@@ -150,6 +151,7 @@ std::vector<WsItem> workspace_items(const et_config_t& c, size_t batch, size_t s
       {I(&ws.lens_scratch), batch * 4},
       {I(&ws.attn_plan), attention_plan_ints(static_cast<int>(batch), static_cast<int>(cap)) * 4},
       {I(&ws.pos_row), cap * 4},
+      {reinterpret_cast<void**>(&ws.mask_bits), f32 ? 0 : attention_mask_bits_words(cap) * 4},
       {F(&ws.a_hi), f32 ? cap * H * 4 : 0}, {F(&ws.a_lo), f32 ? cap * H * 4 : 0},
       {F(&ws.ffn_lo), f32 ? cap * f * 4 : 0},
       {I(&ws.ln_counters), ln_counter_ints(bs) * 4},
@@ -214,6 +216,7 @@ struct et_handle_s {
   const void* cur_attr_mask = nullptr;
   const int* cur_word_idx = nullptr;
   const int* cur_batch_idx = nullptr;
+  bool mask_bits_ready = false;  // ws.mask_bits holds that mask (inside a whole-stack call)
   std::vector<LayerWeights> layers;
   ModelWeights model;
   Workspace ws;
@@ -339,6 +342,7 @@ struct MaskScope {
     h->cur_attr_mask = nullptr;
     h->cur_batch_idx = nullptr;
     h->cur_word_idx = nullptr;
+    h->mask_bits_ready = false;
   }
 };
 
@@ -511,7 +515,7 @@ int run_layer(et_handle_t h, const LayerWeights& lw, const T* x_in, T* x_out, co
                                        reinterpret_cast<__half*>(ctx), ws.attn_plan, batch, max_m, heads, d,
                                        ws.status, s, turn(), &h->maps,
                                        static_cast<const __half*>(h->cur_attr_mask), h->cur_batch_idx,
-                                       h->cur_word_idx, seq));
+                                       h->cur_word_idx, seq, h->mask_bits_ready ? ws.mask_bits : nullptr));
   else if (masked)
     ET_LAUNCH(h, ET_PROF_ATTENTION, 1, s,
               launch_attention_masked_simt<T>(qkv, qkv + hid, qkv + 2 * hid, 3LL * hid, d, ctx,
@@ -734,7 +738,13 @@ int stack_impl(et_handle_t h, int batch, int seq, cudaStream_t s) {
   if (tiles)  // the packed-tile attention serves key-only and general masks
     ET_LAUNCH(h, ET_PROF_PADDING_OFFSETS, 1, s,
               launch_attention_plan(ws.cu_seqlens, batch, max_m, ws.attn_plan, s));
-  else if (h->cur_attr_mask != nullptr)
+  if (tiles && h->cur_attr_mask != nullptr) {
+    ET_LAUNCH(h, ET_PROF_PADDING_OFFSETS, 1, s,
+              launch_attention_mask_bits(static_cast<const __half*>(h->cur_attr_mask), h->cur_batch_idx,
+                                         h->cur_word_idx, ws.cu_seqlens, ws.valid_word_num, max_m, seq, ws.mask_bits,
+                                         s));
+    h->mask_bits_ready = true;  // (MaskScope, which set the mask, clears it)
+  } else if (!tiles && h->cur_attr_mask != nullptr)
     ET_LAUNCH(h, ET_PROF_PADDING_OFFSETS, 1, s,
               launch_position_rows(ws.batch_idx, ws.word_idx, ws.valid_word_num, batch, seq, ws.pos_row, s));
   // No LayerNorm between the projections: x holds un-normalised sums from the first layer's end on,

@@ -166,6 +166,37 @@ def test_whole_path_under_a_general_mask(dtype):
 
 
 @pytest.mark.parametrize("prefix", [True, False], ids=["prefix_mask", "mask_with_holes"])
+@pytest.mark.parametrize("seq", [1, 33, 53, 64, 127, 128])
+def test_mask_as_bits_per_token_equals_the_mask_read_in_the_kernel(prefix, seq):
+    """A whole-stack call turns the general mask into bits once per batch; the op-by-op call reads the mask in the
+    attention kernel.  Same predicate per (query, key), so the same bits out, for every kind of mask."""
+    batch, spec = 9, W.tiny_spec(dtype="fp16")
+    sh = spec.shape
+    rng = np.random.RandomState(11 + seq + int(prefix))
+    lens = rng.randint(1, seq + 1, size=batch).astype(np.int32)
+    lens[2], lens[5] = 0, seq
+    mask_np = W.prefix_mask(lens, seq) if prefix else (rng.rand(batch, seq) < 0.7).astype(np.int32)
+    wl = W.make_workload(spec, random_gamma_beta=True)
+    eng = et.EffectiveTransformer(sh.num_layers, sh.head_num, sh.size_per_head, sh.ffn_dim, batch, seq,
+                                  dtype=torch.float16)
+    eng.set_weights(wl.weights)
+    x = dev(rng.randn(batch, seq, sh.hidden).astype(np.float32), torch.float16)
+    m = dev(mask_np)
+    cfg = et.BertConfig(sh.hidden, sh.num_layers, sh.head_num, sh.ffn_dim)
+    masks = {"random": (rng.rand(batch, seq, seq) < 0.5).astype(np.float32),
+             "causal": np.tril(np.ones((batch, seq, seq), np.float32)),
+             "nothing": np.zeros((batch, seq, seq), np.float32), "all": np.ones((batch, seq, seq), np.float32)}
+    for name, am_np in masks.items():
+        am = dev(am_np, torch.float16)
+        whole = eng.forward_general_mask(x, m, am)
+        eng.set_general_mask(True)
+        ops = et.get_sequence_output(cfg, batch, seq, am, m, x, wl.weights, engine=eng)
+        eng.set_general_mask(False)
+        assert torch.equal(whole, ops), name
+    eng.close()
+
+
+@pytest.mark.parametrize("prefix", [True, False], ids=["prefix_mask", "mask_with_holes"])
 @pytest.mark.parametrize("seq", [64, 128, 40])
 def test_general_mask_attention_on_tensor_cores(prefix, seq):
     """et_attention_tiles_general_mask (the packed-tile tcgen05 kernel reading the mask per query and
