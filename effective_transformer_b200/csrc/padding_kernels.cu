@@ -158,30 +158,48 @@ remove_padding_kernel(const char* __restrict__ from, const int* __restrict__ bat
 
 // One pass over the padded output: item v < T copies packed row v to its
 // padded row and zero-fills the gap of padded rows in front of it; item T
-// zero-fills everything behind the last valid row.
+// zero-fills everything behind the last valid row.  A CTA takes a contiguous run
+// of items and shares their gaps out row by row among its warps: with a warp per
+// item, the warp in front of a short sequence's padding filled all of it alone
+// (32 x 512 positions, gaps of up to 448 rows: 51.7 us under ncu for 39 MB).
 __global__ void __launch_bounds__(kCopyWarpsPerCta * 32)
 restore_padding_kernel(const char* __restrict__ from, const int* __restrict__ batch_idx,
                        const int* __restrict__ word_idx, const int* __restrict__ t_ptr,
                        char* __restrict__ to, int max_rows, int seq, int row_bytes) {
+  constexpr int kItems = kCopyWarpsPerCta * 32;
+  __shared__ int gap_lo[kItems], gap_hi[kItems];  // padded rows [lo, hi) in front of an item; hi = the item's own row
   pdl_wait();
   pdl_trigger();
   int t = *t_ptr;
   t = t < 0 ? 0 : (t > max_rows ? max_rows : t);
-  const int lane = threadIdx.x & 31;
-  const int warp = blockIdx.x * kCopyWarpsPerCta + (threadIdx.x >> 5);
-  const int nwarps = gridDim.x * kCopyWarpsPerCta;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int nvec = row_bytes >> 4;
-  for (int v = warp; v <= t; v += nwarps) {
-    long long prev = -1, cur = max_rows;
-    if (v > 0) prev = static_cast<long long>(batch_idx[v - 1]) * seq + word_idx[v - 1];
-    if (v < t) cur = static_cast<long long>(batch_idx[v]) * seq + word_idx[v];
-    if (prev < -1 || prev >= max_rows) prev = max_rows;  // corrupt index: nothing to fill
-    if (cur < 0 || cur > max_rows) cur = max_rows;
-    for (long long r = prev + 1; r < cur; ++r)
-      warp_zero_row(to + static_cast<size_t>(r) * row_bytes, nvec, lane);
-    if (v < t && cur < max_rows)
-      warp_copy_row<4>(from + static_cast<size_t>(v) * row_bytes,
-                       to + static_cast<size_t>(cur) * row_bytes, nvec, lane);
+  const int per_cta = t / static_cast<int>(gridDim.x) + 1;  // of t + 1 items
+  const long long first = static_cast<long long>(blockIdx.x) * per_cta;
+  const int last = static_cast<int>(min(first + per_cta, static_cast<long long>(t) + 1));
+  for (int base = static_cast<int>(min(first, static_cast<long long>(last))); base < last; base += kItems) {
+    const int n = min(kItems, last - base);
+    if (static_cast<int>(threadIdx.x) < n) {
+      const int v = base + threadIdx.x;
+      long long prev = -1, cur = max_rows;
+      if (v > 0) prev = static_cast<long long>(batch_idx[v - 1]) * seq + word_idx[v - 1];
+      if (v < t) cur = static_cast<long long>(batch_idx[v]) * seq + word_idx[v];
+      if (prev < -1 || prev >= max_rows) prev = max_rows;  // corrupt index: nothing to fill
+      if (cur < 0 || cur > max_rows) cur = max_rows;
+      gap_lo[threadIdx.x] = static_cast<int>(prev + 1);
+      gap_hi[threadIdx.x] = static_cast<int>(cur);
+    }
+    __syncthreads();
+    for (int e = 0; e < n; ++e)
+      for (int r = gap_lo[e] + ((warp + e) & (kCopyWarpsPerCta - 1)); r < gap_hi[e]; r += kCopyWarpsPerCta)
+        warp_zero_row(to + static_cast<size_t>(r) * row_bytes, nvec, lane);
+    for (int e = warp; e < n; e += kCopyWarpsPerCta) {
+      const int v = base + e, cur = gap_hi[e];
+      if (v < t && cur < max_rows)
+        warp_copy_row<4>(from + static_cast<size_t>(v) * row_bytes, to + static_cast<size_t>(cur) * row_bytes, nvec,
+                         lane);
+    }
+    __syncthreads();  // the gaps are rewritten by the next run of items
   }
 }
 

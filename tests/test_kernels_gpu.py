@@ -102,6 +102,23 @@ def test_restore_padding_all_padding_and_no_padding():
         assert torch.equal(out, x * fill)
 
 
+@pytest.mark.parametrize("lens,s", [([1, 512, 0, 0, 3, 511], 512), ([0, 0, 7], 700), ([40] * 300, 41), ([2] * 5000, 3)])
+def test_restore_padding_long_gaps(lens, s):
+    """Gaps longer than a CTA's warps, empty sequences side by side, more items than a CTA holds at once."""
+    b, h = len(lens), 128
+    mask = (np.arange(s)[None] < np.asarray(lens)[:, None]).astype(np.int32)
+    idx = padding_offsets(dev(mask))
+    t = int(sum(lens))
+    packed = torch.randn(max(t, 1), h, device="cuda", dtype=torch.float16)
+    out = torch.full((b, s, h), 7.0, device="cuda", dtype=torch.float16)
+    ok(lib().et_restore_padding(_capi.ET_FP16, iptr(packed), iptr(idx["batch_idx"]), iptr(idx["word_idx"]),
+                                iptr(idx["valid_word_num"]), iptr(out), b, s, h, stream()))
+    torch.cuda.synchronize()
+    want = torch.zeros_like(out)
+    want[torch.from_numpy(mask).bool().cuda()] = packed[:t]
+    assert torch.equal(out, want)
+
+
 def _tol(dtype):
     # one rounding of an O(1..10) value in the output type
     return dict(rtol=2e-3, atol=2e-3) if dtype == torch.float16 else dict(rtol=2e-5, atol=2e-5)
