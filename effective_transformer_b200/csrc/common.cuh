@@ -413,7 +413,7 @@ cudaError_t launch_gemm_tcgen05(const __half* a, const __half* w_packed, const _
                                 int* status_word, cudaStream_t stream, bool reverse_m = false,
                                 const __half* residual = nullptr, TensorMapCache* maps = nullptr,
                                 const GemmLayerNorm* ln = nullptr, bool weights_ready = false);
-// Projections of small batches on tiles of 128 x 64 whose K range is split over a cluster
+// Projections of small batches on tiles of 128 x 64 (fp32 also 128 x 128) whose K range is split over a cluster
 // (gemm_split.cu).  fp16: a [max_m,k], w [n,k], c fp16.  a_lo / w_lo given: fp32 by the three-product tf32
 // split, c_lo as in launch_gemm_tf32x3.
 struct SplitGemm {
@@ -431,9 +431,15 @@ struct SplitGemm {
   int* status_word = nullptr;
   GemmLayerNorm ln;
 };
-// How many CTAs share a tile's K range, or 0 where the persistent kernels serve the shape better.
-int gemm_split_count(int max_m, int n, int k, bool tf32);
-cudaError_t launch_gemm_split(const SplitGemm& g, int epilogue, int splits, TensorMapCache* maps, cudaStream_t stream);
+// Tile width and how many CTAs share a tile's K range; splits 0 where the persistent kernels serve the shape
+// better.
+struct SplitPlan {
+  int bn = 64;
+  int splits = 0;
+};
+SplitPlan gemm_split_plan(int max_m, int n, int k, bool tf32);
+cudaError_t launch_gemm_split(const SplitGemm& g, int epilogue, const SplitPlan& plan, TensorMapCache* maps,
+                              cudaStream_t stream);
 // Whether the fused LayerNorm epilogues can serve a projection of n output columns.
 inline bool gemm_layernorm_supported(int n) { return n > 0 && n % 256 == 0 && n <= 1024; }
 

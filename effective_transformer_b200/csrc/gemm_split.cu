@@ -5,14 +5,15 @@
 // of K: right when there are tiles for every SM, but a batch of a few hundred tokens has 3 to 24 of them,
 // and each walks K alone (48 dependent 64-wide steps for K = 3072) while most of the GPU idles.  What
 // bounds such a projection is the latency of that chain and how many SMs pull on the weights (1 to 5 MB).
-// So here a tile is 128 x 64 and its K range is cut into `splits` (1, 2, 4 or 8) parts, one CTA each:
-//   warp 0      TMA producer: A [128 x BK] and W [64 x BK] boxes into a ring of shared-memory stages
-//   warp 1      tcgen05.mma (M = 128, N = 64) into TMEM, one accumulator block per accumulation unit
+// So here a tile is 128 x 64 (fp32 also 128 x 128: a third less to fetch per output, where the number of CTAs
+// that run at once, one per SM, is the limit) and its K range is cut into `splits` (1 to 8) parts, one CTA each:
+//   warp 0      TMA producer: A [128 x BK] and W [64 or 128 x BK] boxes into a ring of shared-memory stages
+//   warp 1      tcgen05.mma (M = 128, N = 64 or 128) into TMEM, one accumulator block per accumulation unit
 //   warps 2-5   read the partial sums from TMEM and send row r to the CTA r % splits of the cluster through
 //               distributed shared memory; behind a cluster barrier each CTA adds the parts of its rows
 //               in rank order (the result does not depend on timing), applies the epilogue and stores
 // Rows are dealt to the CTAs by r % splits, so a last tile with few rows still keeps all of them busy.
-// The shared memory of a CTA is below half an SM's, so the next projection's CTAs are resident while this
+// The shared memory of an fp16 CTA is below half an SM's, so the next projection's CTAs are resident while this
 // one runs, and the producer requests their W boxes before it waits for this kernel
 // (`weights_ready`: W was complete before the preceding kernel began): a weight's trip from HBM then lies
 // under the kernel before.  Every mbarrier wait is bounded.
@@ -28,7 +29,6 @@ namespace {
 using namespace ptx;
 
 constexpr int BM = 128;
-constexpr int BN = 64;
 constexpr int kRowBytes = 128;        // one swizzle row of an operand tile: 64 fp16 or 32 tf32
 constexpr int kThreads = 192;
 constexpr int kEpThreads = 128;
@@ -36,8 +36,9 @@ constexpr int kMaxSplits = 8;
 
 enum Site : int { kSiteProducer = 1, kSiteDrain = 2, kSiteMma = 3, kSiteMmaDrain = 4, kSiteEpilogue = 5, kSiteAlign = 6 };
 
-template <bool kTf32>
+template <bool kTf32, int BN>
 struct Cfg {
+  static constexpr bool kWide = BN == 128;
   static constexpr int BK = kTf32 ? 32 : 64;
   static constexpr int kParts = kTf32 ? 2 : 1;  // tf32: hi and lo halves of both operands
   static constexpr int kABytes = BM * kRowBytes;
@@ -47,11 +48,18 @@ struct Cfg {
   // tf32: the tensor core adds into its accumulator with truncation, so a chain is cut every six k-blocks
   // (see gemm_tf32x3.cu); every unit has a TMEM block of its own here.  fp16: one unit.
   static constexpr int kUnitKb = kTf32 ? 6 : 1 << 20;
-  static constexpr int kBlocks = kTf32 ? 8 : 1;
+  static constexpr int kBlocks = kTf32 ? 512 / BN : 1;
   static constexpr int kTmemCols = kBlocks * BN;
-  static constexpr int kRecvBytes = BM * BN * 4;
+  // partial sums of this CTA's rows from every CTA of the cluster: splits * ceil(128 / splits) rows.  The 128-wide
+  // tiles receive them where their operand stages were: both would not fit an SM.
+  static constexpr int kRecvBytes = (BM + kMaxSplits) * BN * 4;
+  static constexpr int kRecvAt = kWide ? 0 : kStages * kStageBytes;
+  static_assert(!kWide || kRecvBytes <= kStages * kStageBytes, "the partial sums must fit the stages");
+  static constexpr int kBarsAt = kWide ? kStages * kStageBytes : kRecvAt + kRecvBytes;
+  static constexpr int kPieces = BN / 8;                // eight-column pieces of a row
+  static constexpr int kRowsPass = kEpThreads / kPieces;  // rows the epilogue threads cover at once
   static constexpr int kNumBars = 2 * kStages + 2;
-  static constexpr int kSmemBytes = kStages * kStageBytes + kRecvBytes + 128;
+  static constexpr int kSmemBytes = kBarsAt + 128;
 };
 
 __device__ __forceinline__ void umma_tf32_ss(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
@@ -99,12 +107,12 @@ struct Maps {
   CUtensorMap a, w, a_lo, w_lo;  // the lo halves only for tf32
 };
 
-template <bool kTf32, int EPI>
+template <bool kTf32, int BN, int EPI>
 __global__ void __launch_bounds__(kThreads, kTf32 ? 1 : 2)
 gemm_split_kernel(const __grid_constant__ Maps maps, void* __restrict__ c_ptr, float* __restrict__ c_lo,
                   const void* __restrict__ bias_ptr, const void* __restrict__ res_ptr, const int* __restrict__ m_ptr,
                   int max_m, int N, int num_kb, int weights_ready, int* status_word, const GemmLayerNorm ln) {
-  using cfg = Cfg<kTf32>;
+  using cfg = Cfg<kTf32, BN>;
   using T = typename std::conditional<kTf32, float, __half>::type;
   constexpr int S = cfg::kStages;
   constexpr bool kNormIn = EPI == kEpiNormIn || EPI == kEpiNormInGelu;
@@ -119,12 +127,13 @@ gemm_split_kernel(const __grid_constant__ Maps maps, void* __restrict__ c_ptr, f
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   const uint32_t base = smem_u32(smem_raw);
   const bool aligned = (base & 1023u) == 0u;  // the same in every CTA of the grid
-  const uint32_t recv = base + S * cfg::kStageBytes;
-  const uint32_t bar0 = recv + cfg::kRecvBytes;
+  const uint32_t recv = base + cfg::kRecvAt;
+  const int slots = (BM + splits - 1) / splits;  // rows of the tile that are this CTA's
+  const uint32_t bar0 = base + cfg::kBarsAt;
   auto full_bar = [&](int s) { return bar0 + 8u * s; };
   auto empty_bar = [&](int s) { return bar0 + 8u * (S + s); };
   const uint32_t acc_bar = bar0 + 8u * (2 * S), drain_bar = acc_bar + 8u;
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem_raw + S * cfg::kStageBytes + cfg::kRecvBytes + 8 * cfg::kNumBars);
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem_raw + cfg::kBarsAt + 8 * cfg::kNumBars);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 
@@ -147,8 +156,9 @@ gemm_split_kernel(const __grid_constant__ Maps maps, void* __restrict__ c_ptr, f
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
-  // every CTA of the cluster runs from here on: its shared memory may be written once all have arrived
-  if (splits > 1) cluster_arrive();
+  // First arrival at the cluster's barrier, behind which the shared memory of its CTAs may be written: every CTA
+  // runs from here on; where the partial sums take the place of the stages, only when its MMAs are done.
+  if (!cfg::kWide && splits > 1) cluster_arrive();
 
   auto fail = [&](int site) {
     *abort_flag = 1;
@@ -211,6 +221,7 @@ gemm_split_kernel(const __grid_constant__ Maps maps, void* __restrict__ c_ptr, f
     }
     __syncwarp();
     if (splits > 1) {
+      if (cfg::kWide) cluster_arrive();
       cluster_wait();
       cluster_arrive();
       cluster_wait();
@@ -253,6 +264,7 @@ gemm_split_kernel(const __grid_constant__ Maps maps, void* __restrict__ c_ptr, f
     }
     __syncwarp();
     if (splits > 1) {
+      if (cfg::kWide) cluster_arrive();
       cluster_wait();
       cluster_arrive();
       cluster_wait();
@@ -260,14 +272,16 @@ gemm_split_kernel(const __grid_constant__ Maps maps, void* __restrict__ c_ptr, f
   } else {
     // ------------------------- partial sums, reduction, epilogue -------------------------
     pdl_wait();
-    const int rows = valid_rows();
+    const int rows = min(valid_rows(), BM);
     const bool live = rows > 0 && aligned;
     const int quad = warp & 3;
     const int t = threadIdx.x - 64;      // 0..127
-    const int piece = t & 7;             // this thread's eight columns
+    const int piece = t % cfg::kPieces;  // this thread's eight columns
     const int col = n0 + piece * 8;
-    const int items = 8 / splits;        // rows of this thread: rank + splits * ((t >> 3) + 16 * j)
-    auto row_of = [&](int j) { return rank + splits * ((t >> 3) + 16 * j); };
+    // slots (rows) of this thread, at most eight: a 128-wide tile has two CTAs at least
+    const int items = (slots + cfg::kRowsPass - 1) / cfg::kRowsPass;
+    auto slot_of = [&](int j) { return t / cfg::kPieces + cfg::kRowsPass * j; };
+    auto row_of = [&](int j) { return rank + splits * slot_of(j); };
     T* C = static_cast<T*>(c_ptr);
     const T* bias = static_cast<const T*>(bias_ptr);
     const T* residual = static_cast<const T*>(res_ptr);
@@ -295,8 +309,8 @@ gemm_split_kernel(const __grid_constant__ Maps maps, void* __restrict__ c_ptr, f
             st[j][0] = st[j][1] = make_float2(0.f, 0.f);
             if (ln.stats_in != nullptr) {
               const float2* sp = reinterpret_cast<const float2*>(ln.stats_in) + static_cast<size_t>(m0 + row_of(j)) * ln.stat_slots;
-              if (piece < ln.stat_slots) st[j][0] = sp[piece];
-              if (piece + 8 < ln.stat_slots) st[j][1] = sp[piece + 8];
+              if ((piece & 7) < ln.stat_slots) st[j][0] = sp[piece & 7];
+              if ((piece & 7) + 8 < ln.stat_slots) st[j][1] = sp[(piece & 7) + 8];
             }
           }
         }
@@ -307,16 +321,19 @@ gemm_split_kernel(const __grid_constant__ Maps maps, void* __restrict__ c_ptr, f
       got = __all_sync(0xffffffffu, mbar_wait(acc_bar, 0u, abort_flag));
       if (!got && lane == 0) fail(kSiteEpilogue);
     }
-    if (splits > 1) cluster_wait();  // (the first arrival: every CTA has started)
+    if (splits > 1) {
+      if (cfg::kWide) cluster_arrive();
+      cluster_wait();
+    }
     if (got && quad * 32 < rows) {
       tc_fence_after();
       const uint32_t t_row = tmem_base + (static_cast<uint32_t>(quad * 32) << 16);
       const int r = quad * 32 + lane;
       const int slot = r / splits;
-      const uint32_t dst0 = recv + ((rank * (BM / splits) + slot) * BN) * 4;
+      const uint32_t dst0 = recv + ((rank * slots + slot) * BN) * 4;
       const uint32_t dst = splits > 1 ? mapa_shared(dst0, r % splits) : dst0;
 #pragma unroll
-      for (int hcol = 0; hcol < 2; ++hcol) {
+      for (int hcol = 0; hcol < BN / 32; ++hcol) {
         float sum[32];
 #pragma unroll
         for (int e = 0; e < 32; ++e) sum[e] = 0.f;
@@ -352,14 +369,14 @@ gemm_split_kernel(const __grid_constant__ Maps maps, void* __restrict__ c_ptr, f
       for (int j = 0; j < 8; ++j) {
         if (j >= items) break;           // uniform
         const int r = row_of(j);
-        const int slot = (t >> 3) + 16 * j;
-        const bool mine = r < rows;      // uniform in the eight lanes of a row
+        const int slot = slot_of(j);
+        const bool mine = r < rows;      // uniform in the lanes of a row
         float f[8];
 #pragma unroll
         for (int e = 0; e < 8; ++e) f[e] = 0.f;
         if (mine) {
           for (int src = 0; src < splits; ++src) {
-            const uint32_t rowp = recv + ((src * (BM / splits) + slot) * BN) * 4;
+            const uint32_t rowp = recv + ((src * slots + slot) * BN) * 4;
             const float4 p0 = ld_shared_f4(rowp + (((2 * piece) ^ (slot & 15)) << 4));
             const float4 p1 = ld_shared_f4(rowp + (((2 * piece + 1) ^ (slot & 15)) << 4));
             f[0] += p0.x, f[1] += p0.y, f[2] += p0.z, f[3] += p0.w;
@@ -451,8 +468,8 @@ gemm_split_kernel(const __grid_constant__ Maps maps, void* __restrict__ c_ptr, f
               a += __shfl_xor_sync(0xffffffffu, a, o2);
               b += __shfl_xor_sync(0xffffffffu, b, o2);
             }
-            if (mine && piece == 0)
-              reinterpret_cast<float2*>(ln.stats_out)[static_cast<size_t>(m0 + r) * (N / 64) + blockIdx.y] = make_float2(a, b);
+            if (mine && (piece & 7) == 0)
+              reinterpret_cast<float2*>(ln.stats_out)[static_cast<size_t>(m0 + r) * (N / 64) + col / 64] = make_float2(a, b);
           }
         }
       }
@@ -468,12 +485,12 @@ gemm_split_kernel(const __grid_constant__ Maps maps, void* __restrict__ c_ptr, f
   }
 }
 
-template <bool kTf32, int EPI>
-cudaError_t launch_split(const Maps& maps, const SplitGemm& g, int splits, cudaStream_t stream) {
-  using cfg = Cfg<kTf32>;
+template <bool kTf32, int BN, int EPI>
+cudaError_t launch_split_bn(const Maps& maps, const SplitGemm& g, int splits, cudaStream_t stream) {
+  using cfg = Cfg<kTf32, BN>;
   static PerDeviceOnce once;  // function attributes are per device
   const cudaError_t once_err = once.run([] {
-    return cudaFuncSetAttribute(gemm_split_kernel<kTf32, EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    return cudaFuncSetAttribute(gemm_split_kernel<kTf32, BN, EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                 cfg::kSmemBytes);
   });
   if (once_err != cudaSuccess) return once_err;
@@ -491,8 +508,15 @@ cudaError_t launch_split(const Maps& maps, const SplitGemm& g, int splits, cudaS
   attr[1].val.programmaticStreamSerializationAllowed = 1;
   lc.attrs = attr;
   lc.numAttrs = pdl_enabled() ? 2 : 1;
-  return cudaLaunchKernelEx(&lc, gemm_split_kernel<kTf32, EPI>, maps, g.c, g.c_lo, g.bias, g.residual, g.m_ptr,
+  return cudaLaunchKernelEx(&lc, gemm_split_kernel<kTf32, BN, EPI>, maps, g.c, g.c_lo, g.bias, g.residual, g.m_ptr,
                             g.max_m, g.n, (g.k + cfg::BK - 1) / cfg::BK, g.weights_ready ? 1 : 0, g.status_word, g.ln);
+}
+
+template <bool kTf32, int EPI>
+cudaError_t launch_split(const Maps& maps, const SplitGemm& g, const SplitPlan& p, cudaStream_t stream) {
+  if constexpr (kTf32)
+    if (p.bn == 128) return launch_split_bn<kTf32, 128, EPI>(maps, g, p.splits, stream);
+  return launch_split_bn<kTf32, 64, EPI>(maps, g, p.splits, stream);
 }
 
 bool encode_split(CUtensorMap* map, bool tf32, const void* base, int rows, int k, int box_rows, TensorMapCache* cache) {
@@ -503,46 +527,78 @@ bool encode_split(CUtensorMap* map, bool tf32, const void* base, int rows, int k
 }  // namespace
 
 // Where a cluster's split pays, from the capacity in rows (the valid rows are only known on the device).
-// One B200, us per launch, rows = 0.6 * capacity, 1 / 2 / 4 / 8 CTAs per tile against the persistent kernel:
-//   fp16, N x K     capacity 64                      512                            2048
-//   768 x 768       6.9  5.1  4.1  4.4 (7.9)         8.2  6.8  7.4 10.2 ( 8.5)      8.7  9.3  17  34 ( 8.7)
-//   2304 x 768      7.2  5.3  5.4  9.1 (8.2)         8.5  7.9 14.4 26.8 ( 9.1)     16.8 25.1  50  98 (10.1)
-//   768 x 3072     17.3 10.3  6.8  5.6 (18.6)       19.5 12.4 10.2 13.1 (19.5)     20.2 14.3  24  42 (20.1)
-//   fp32, N x K
-//   2304 x 768     17.9 11.0 14.7 17.9 (17.4)       19.6 23.2 32.7 57.9 (17.7)
-//   768 x 3072     55.1 30.3 17.1 11.1 (55.1)       54.7 31.8 34.3 34.4 (54.6)
-// So: as many CTAs per tile as still run at once (two fp16 CTAs per SM, one fp32), each with enough of K to
-// hide its load latency: six 64-wide or twelve 32-wide steps, or three where the grid is small enough (two
-// thirds of the SMs) not to share L2 bandwidth.  From six row tiles on a third more CTAs than run at once is
-// taken, if their share of K is long: a batch has padding, and the tiles it leaves empty cost next to nothing.
-int gemm_split_count(int max_m, int n, int k, bool tf32) {
-  if (n % BN != 0 || max_m <= 0) return 0;
+// One B200, us per launch with 60 % / 100 % of the capacity valid; "64x4" = tiles 64 wide, 4 CTAs per tile; the
+// persistent kernels in brackets:
+//   fp16, N x K   capacity 64           512                                  2048
+//   768 x 768     64x4 4.1/4.5 (7.9)    64x2 6.4/6.3   64x4 7.4/7.7 (8.6)    64x1 7.9/8.3  64x2 9.0/13.8 (8.8)
+//   2304 x 768    64x2 5.2/5.5 (8.2)    64x2 7.5/8.1   64x3 11.8    (9.1)    64x1 15.5                   (10.1)
+//   768 x 3072    64x8 5.5/6.1 (18.6)   64x4 10.2/11.0 64x8 13/17   (19.5)   64x2 14.0/25.3 64x3 21.1    (20.0)
+//   fp32, N x K   capacity 64           256                                  512
+//   768 x 768     64x8 5.6/5.8 (15.9)   64x4 8.4/8.6   128x8 9.8/10.1 (16.3) 64x2 11.4/11.7 128x5 11.4/11.9 (16.4)
+//   3072 x 768    128x5 10.0/11.1 (19.8) 64x2 21.6/24.6 128x2 16.3/16.7 (19.9) 128x2 17.7/30.6              (20.6)
+//   768 x 3072    64x8 11.1/11.4 (55.1) 64x4 18.8/19.0 128x8 15.9/16.1 (54.7) 64x2 31.6/32.0 128x5 20.6/20.9 (54.4)
+// fp16: the most CTAs per tile with six 64-wide steps of K each to hide the load latency, or three where the grid
+// is small enough (two thirds of the SMs) not to share L2 bandwidth.  Two CTAs fit an SM, but clusters of more
+// than two stop finding places on a third more CTAs than SMs.
+// fp32: one CTA fits an SM; among the plans whose clusters all find one (clusters of more than two: 85 % of the
+// SMs) the one whose CTA fetches the least, 64 or 48 KB per 32-wide step, a 128-wide tile's longer reduction counted as
+// another 128 KB.
+// From six row tiles on a third more CTAs than run at once is taken, if their share of K is long (12 or, fp32, 24
+// steps): a batch has
+// padding, and the tiles it leaves empty cost next to nothing.
+SplitPlan gemm_split_plan(int max_m, int n, int k, bool tf32) {
+  SplitPlan best;
+  if (max_m <= 0) return best;
   const int num_kb = (k + (tf32 ? 31 : 63)) / (tf32 ? 32 : 64);
-  const long long m_tiles = (max_m + BM - 1) / BM, tiles = m_tiles * (n / BN);
-  const long long sms = sm_count(), at_once = sms * (tf32 ? 1 : 2);
-  for (int splits = kMaxSplits; splits >= 1; splits >>= 1) {
-    const int share = num_kb / splits;
-    const long long ctas = tiles * splits;
-    if (share < 1 || (tf32 && (num_kb + splits - 1) / splits > Cfg<true>::kBlocks * Cfg<true>::kUnitKb)) continue;
-    if (splits == 1) return tf32 || ctas > at_once ? 0 : 1;  // fp32: no better than the 128 x 128 tiles
-    if (share < 3 || (share < (tf32 ? 12 : 6) && 3 * ctas > 2 * sms)) continue;
-    if (ctas <= at_once || (m_tiles >= 6 && share >= 12 && 3 * ctas <= 4 * at_once)) return splits;
+  const long long m_tiles = (max_m + BM - 1) / BM, sms = sm_count();
+  const bool padded = m_tiles >= 6;
+  if (!tf32) {
+    const long long tiles = m_tiles * (n / 64);
+    if (n % 64 != 0) return best;
+    for (int splits = kMaxSplits; splits >= 1 && best.splits == 0; splits >>= 1) {
+      const int share = num_kb / splits;
+      const long long ctas = tiles * splits;
+      if (share < 1 || (splits > 1 && (share < 3 || (share < 6 && 3 * ctas > 2 * sms)))) continue;
+      if (splits > 2 ? 3 * ctas <= 4 * sms
+                     : ctas <= 2 * sms || (splits == 2 && padded && share >= 12 && 3 * ctas <= 8 * sms))
+        best.splits = splits;
+    }
+    return best;
   }
-  return 0;
+  constexpr int kCounts[] = {2, 3, 4, 5, 6, 8};
+  for (const bool second_try : {false, true}) {
+    int least = 0;
+    for (const int bn : {64, 128}) {
+      if (n % bn != 0) continue;
+      for (const int splits : kCounts) {
+        const int share = (num_kb + splits - 1) / splits;
+        const long long ctas = m_tiles * (n / bn) * splits;
+        const int most = bn == 64 ? Cfg<true, 64>::kBlocks * Cfg<true, 64>::kUnitKb
+                                  : Cfg<true, 128>::kBlocks * Cfg<true, 128>::kUnitKb;  // what TMEM holds
+        if (num_kb / splits < 3 || share > most) continue;
+        if (second_try ? !(padded && share >= 24 && 3 * ctas <= 4 * sms) : 20 * ctas > (splits > 2 ? 17 : 20) * sms)
+          continue;
+        const int fetched = bn == 64 ? share * 48 : share * 64 + 128;
+        if (best.splits == 0 || fetched < least) best.bn = bn, best.splits = splits, least = fetched;
+      }
+    }
+    if (best.splits != 0) break;
+  }
+  return best;
 }
 
-cudaError_t launch_gemm_split(const SplitGemm& g, int epilogue, int splits, TensorMapCache* maps, cudaStream_t stream) {
+cudaError_t launch_gemm_split(const SplitGemm& g, int epilogue, const SplitPlan& plan, TensorMapCache* maps, cudaStream_t stream) {
   const bool tf32 = g.a_lo != nullptr;
   Maps m;
-  if (!encode_split(&m.a, tf32, g.a, g.max_m, g.k, BM, maps) || !encode_split(&m.w, tf32, g.w, g.n, g.k, BN, maps))
+  if (!encode_split(&m.a, tf32, g.a, g.max_m, g.k, BM, maps) || !encode_split(&m.w, tf32, g.w, g.n, g.k, plan.bn, maps))
     return cudaErrorInvalidValue;
   m.a_lo = m.a, m.w_lo = m.w;
   if (tf32 && (!encode_split(&m.a_lo, true, g.a_lo, g.max_m, g.k, BM, maps) ||
-               !encode_split(&m.w_lo, true, g.w_lo, g.n, g.k, BN, maps)))
+               !encode_split(&m.w_lo, true, g.w_lo, g.n, g.k, plan.bn, maps)))
     return cudaErrorInvalidValue;
 #define ETB_CASE(TF, E) \
   case E:               \
-    return launch_split<TF, E>(m, g, splits, stream)
+    return launch_split<TF, E>(m, g, plan, stream)
   if (tf32) {
     switch (epilogue) {
       ETB_CASE(true, kEpiNone);

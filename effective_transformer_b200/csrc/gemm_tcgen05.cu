@@ -1359,14 +1359,14 @@ cudaError_t launch_gemm_tcgen05(const __half* a, const __half* w_packed, const _
     }
     lnp = *ln;
   }
-  if (const int splits = has_ln(epilogue) ? 0 : gemm_split_count(max_m, n, k, false)) {
+  if (const SplitPlan plan = has_ln(epilogue) ? SplitPlan() : gemm_split_plan(max_m, n, k, false); plan.splits != 0) {
     SplitGemm g;
     g.a = a, g.w = w_packed, g.bias = bias, g.residual = residual, g.c = c;
     g.m_ptr = m_ptr, g.max_m = max_m, g.n = n, g.k = k;
     g.weights_ready = weights_ready;
     g.status_word = status_word;
     g.ln = lnp;
-    return launch_gemm_split(g, epilogue, splits, maps, stream);
+    return launch_gemm_split(g, epilogue, plan, maps, stream);
   }
   const int bn = (n % 256 == 0) ? 256 : 128;
   const bool pair = bn == 256;

@@ -816,13 +816,13 @@ cudaError_t launch_gemm_tf32x3(const float* a_hi, const float* a_lo, const float
   if (bias != nullptr && (reinterpret_cast<uintptr_t>(bias) & 15u)) return cudaErrorMisalignedAddress;
   if (c_lo != nullptr && (reinterpret_cast<uintptr_t>(c_lo) & 15u)) return cudaErrorMisalignedAddress;
   if (epilogue != kEpiNone && bias == nullptr) return cudaErrorInvalidValue;
-  if (const int splits = gemm_split_count(max_m, n, k, true)) {
+  if (const SplitPlan plan = gemm_split_plan(max_m, n, k, true); plan.splits != 0) {
     SplitGemm g;
     g.a = a_hi, g.a_lo = a_lo, g.w = w_hi, g.w_lo = w_lo, g.bias = bias, g.c = c, g.c_lo = c_lo;
     g.m_ptr = m_ptr, g.max_m = max_m, g.n = n, g.k = k;
     g.weights_ready = weights_ready;
     g.status_word = status_word;
-    return launch_gemm_split(g, epilogue, splits, maps, stream);
+    return launch_gemm_split(g, epilogue, plan, maps, stream);
   }
   CUtensorMap tah, tal, twh, twl;
   if (!encode_2d_f32_sw128(&tah, a_hi, static_cast<uint64_t>(max_m), static_cast<uint64_t>(k), BM, maps) ||

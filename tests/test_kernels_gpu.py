@@ -449,12 +449,13 @@ def test_gemm_fp32_on_tensor_cores_keeps_fp32_accuracy(m, cap, n, k, epi):
         assert float((one_term - plain).abs().max()) > 20 * float((c[:m].double() - ref).abs().max()) or k < 128
 
 
-# Small batches, whose projections split a tile's K range over a cluster (1, 2, 4 and 8 CTAs per tile):
-# fewer rows than CTAs, a row tile's edges, a last tile with one row, a row tile the batch leaves empty, K that
+# Small batches, whose projections split a tile's K range over a cluster (1 to 8 CTAs per tile, which
+# need not divide its 128 rows; fp32 tiles 64 and 128 wide): fewer rows than CTAs, a row tile's edges, a last tile with one row, a row tile the batch leaves empty, K that
 # does not divide evenly (or at all: fp16 K of 8), N of an odd number of 64-column tiles per 128.
 SPLIT_SHAPES = [(3, 64, 768, 3072), (127, 128, 768, 768), (128, 128, 2304, 768), (129, 256, 768, 3072),
                 (40, 256, 3072, 768), (385, 700, 768, 3072), (500, 512, 384, 1600), (600, 640, 1024, 4096),
-                (513, 768, 3072, 768)]
+                (513, 768, 3072, 768), (200, 256, 768, 768), (30, 50, 2304, 768), (700, 1024, 768, 3072),
+                (250, 500, 2304, 768)]
 
 
 @pytest.mark.parametrize("m,cap,n,k", SPLIT_SHAPES + [(77, 90, 256, 1000), (5, 8, 128, 72)])
