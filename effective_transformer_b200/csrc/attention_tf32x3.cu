@@ -13,6 +13,9 @@
 // sequence of the reference (tf_op/bert_transformer_op.cu.cc:158-191,
 // cuda/attention.cu:249-492) for OperationType FP32; no padded position is loaded
 // or computed.  Warp w of the four owns query rows [16 w, 16 w + 16) of the tile.
+// The exponentials and stores of 8-key blocks past the sequence's end are skipped, and the outputs are rescaled
+// only from the second key block on: BERT-base, 8 sequences of 8 to 32 tokens, 1046 -> 1025 us per pass (at 500 x 64
+// the pass runs at the power limit and does not change: 17.9 ms).
 #include "common.cuh"
 
 namespace etb {
@@ -161,10 +164,12 @@ attention_tf32x3_kernel(const float* __restrict__ q, const float* __restrict__ k
         float mx = -INFINITY;
 #pragma unroll
         for (int nb = 0; nb < 8; ++nb)
+          if (nb < nkb) {  // (uniform) 8-key blocks past the sequence cost nothing here either
 #pragma unroll
-          for (int e = 0; e < 2; ++e) {
-            if (nb * 8 + 2 * t + e >= nk) s[nb][2 * hh + e] = -INFINITY;
-            mx = fmaxf(mx, s[nb][2 * hh + e]);
+            for (int e = 0; e < 2; ++e) {
+              if (nb * 8 + 2 * t + e >= nk) s[nb][2 * hh + e] = -INFINITY;
+              mx = fmaxf(mx, s[nb][2 * hh + e]);
+            }
           }
         mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 1));
         mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 2));
@@ -174,27 +179,32 @@ attention_tf32x3_kernel(const float* __restrict__ q, const float* __restrict__ k
         float sum = 0.f;
 #pragma unroll
         for (int nb = 0; nb < 8; ++nb)
+          if (nb < nkb) {
 #pragma unroll
-          for (int e = 0; e < 2; ++e) {
-            const float p = expf(s[nb][2 * hh + e] - m_new);
-            s[nb][2 * hh + e] = p;
-            sum += p;
+            for (int e = 0; e < 2; ++e) {
+              const float p = expf(s[nb][2 * hh + e] - m_new);
+              s[nb][2 * hh + e] = p;
+              sum += p;
+            }
           }
         l[hh] = l[hh] * r + sum;  // this lane's share of the row sum
+        if (k0 > 0) {
 #pragma unroll
-        for (int nb = 0; nb < 8; ++nb) {
-          o[nb][2 * hh] *= r;
-          o[nb][2 * hh + 1] *= r;
+          for (int nb = 0; nb < 8; ++nb) {
+            o[nb][2 * hh] *= r;
+            o[nb][2 * hh + 1] *= r;
+          }
         }
       }
     }
     __syncthreads();  // every warp has read its K fragments: the tile becomes the probabilities
     if (active) {
 #pragma unroll
-      for (int nb = 0; nb < 8; ++nb) {
-        *reinterpret_cast<float2*>(&Ks[rw + g][nb * 8 + 2 * t]) = make_float2(s[nb][0], s[nb][1]);
-        *reinterpret_cast<float2*>(&Ks[rw + g + 8][nb * 8 + 2 * t]) = make_float2(s[nb][2], s[nb][3]);
-      }
+      for (int nb = 0; nb < 8; ++nb)
+        if (nb < nkb) {
+          *reinterpret_cast<float2*>(&Ks[rw + g][nb * 8 + 2 * t]) = make_float2(s[nb][0], s[nb][1]);
+          *reinterpret_cast<float2*>(&Ks[rw + g + 8][nb * 8 + 2 * t]) = make_float2(s[nb][2], s[nb][3]);
+        }
       __syncwarp();  // a warp reads back only the probability rows it wrote itself
       // ---- O += P V: one step per 8 keys, 8 blocks of 8 output columns ----
 #pragma unroll 2
