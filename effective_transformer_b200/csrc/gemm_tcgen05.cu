@@ -1139,7 +1139,9 @@ cudaError_t launch_pair_epi(const CUtensorMap& ta, const CUtensorMap& tb, const 
   if (once_err != cudaSuccess) return once_err;
   const long long max_tiles = static_cast<long long>((max_m + 2 * BM - 1) / (2 * BM)) * (n / cfg::BN);
   long long pairs = sm_count() / 2;
-  if (pairs > max_tiles) pairs = max_tiles;
+  // Up to two pairs per tile: when the tiles would occupy at most half of the pairs, pair_units cuts them into
+  // half-width units.  T = 2000, N = 768: 24 tiles on 48 pairs, K = 768 12.1 -> 11.2 us, K = 3072 26.1 -> 24.4 us (ncu).
+  if (pairs > 2 * max_tiles) pairs = 2 * max_tiles;
   if (pairs < 1) pairs = 1;
   return launch_pdl(gemm_tcgen05_pair_kernel<EPI, VPL>, dim3(static_cast<int>(2 * pairs)), dim3(threads_of(EPI)),
                     cfg::kSmemBytes, stream, ta, tb, tbh, c, bias, residual, m_ptr, max_m, n, k, status_word, reverse_m,
