@@ -437,7 +437,7 @@ struct SplitPlan {
   int bn = 64;
   int splits = 0;
 };
-SplitPlan gemm_split_plan(int max_m, int n, int k, bool tf32);
+SplitPlan gemm_split_plan(int max_m, int n, int k, bool tf32, bool feeds_attention = false);
 cudaError_t launch_gemm_split(const SplitGemm& g, int epilogue, const SplitPlan& plan, TensorMapCache* maps,
                               cudaStream_t stream);
 // Whether the fused LayerNorm epilogues can serve a projection of n output columns.

@@ -527,45 +527,52 @@ bool encode_split(CUtensorMap* map, bool tf32, const void* base, int rows, int k
 }  // namespace
 
 // Where a cluster's split pays, from the capacity in rows (the valid rows are only known on the device).
-// One B200, us per launch with 60 % / 100 % of the capacity valid; "64x4" = tiles 64 wide, 4 CTAs per tile; the
-// persistent kernels in brackets:
-//   fp16, N x K   capacity 64           512                                  2048
-//   768 x 768     64x4 4.1/4.5 (7.9)    64x2 6.4/6.3   64x4 7.4/7.7 (8.6)    64x1 7.9/8.3  64x2 9.0/13.8 (8.8)
-//   2304 x 768    64x2 5.2/5.5 (8.2)    64x2 7.5/8.1   64x3 11.8    (9.1)    64x1 15.5                   (10.1)
-//   768 x 3072    64x8 5.5/6.1 (18.6)   64x4 10.2/11.0 64x8 13/17   (19.5)   64x2 14.0/25.3 64x3 21.1    (20.0)
-//   fp32, N x K   capacity 64           256                                  512
-//   768 x 768     64x8 5.6/5.8 (15.9)   64x4 8.4/8.6   128x8 9.8/10.1 (16.3) 64x2 11.4/11.7 128x5 11.4/11.9 (16.4)
-//   3072 x 768    128x5 10.0/11.1 (19.8) 64x2 21.6/24.6 128x2 16.3/16.7 (19.9) 128x2 17.7/30.6              (20.6)
-//   768 x 3072    64x8 11.1/11.4 (55.1) 64x4 18.8/19.0 128x8 15.9/16.1 (54.7) 64x2 31.6/32.0 128x5 20.6/20.9 (54.4)
-// fp16: the most CTAs per tile with six 64-wide steps of K each to hide the load latency, or three where the grid
+// Measured where it counts, inside a replayed pass, whose kernels overlap and whose weights come from HBM: us per
+// pass on one B200 with one projection's plan changed and the others at their best ("64x4" = tiles 64 wide, 4 CTAs
+// per tile; "-" = the persistent kernels).  BERT-base fp16, capacity 64 / 256 / 512 / 1024 / 2048 (60 to 70 % valid):
+//   QKV       64x1 426  64x2 463  - 452    64x2 515 - 489            64x2 543 - 521   64x1 635 - 587   - 706
+//   out       64x4 426  64x2 460  - 467    64x4 490 - 542            64x2 526 - 555   64x2 591 - 608   64x2 733 - 707
+//   FFN1      64x2 425  64x4 471  - 460    64x2 488 - 504            64x2 561 - 517   64x1 638 - 592   - 706
+//   FFN2      64x8 425  64x4 489  - 638    64x8 489 64x4 525 - 647   64x4 530 - 660   64x2 587 - 660   64x2 707 - 734
+// and with every row of 2048 valid FFN2 64x2 919, - 839.  BERT-large at capacity 64: QKV 64x3 848, - 910; FFN1
+// 64x3 854, 64x2 890, - 900.  fp32, BERT-base, capacity 64 / 256 / 512:
+//   QKV       64x3 755  - 853              64x2 949 128x2 981 - 1001  128x2 1223 - 1170
+//   out       64x8 754  - 876              64x5 949 64x4 962 - 1064   128x5 1170 64x2 1173 - 1342
+//   FFN1      128x5 755 64x2 767 - 856     128x2 949 64x2 1005 - 965  128x2 1162 - 1155
+//   FFN2      64x8 755  - 1269             128x8 951 64x4 978 - 1401  128x5 1186 64x2 1295 - 1669
+// fp16: the most CTAs per tile with five 64-wide steps of K each to hide the load latency, or three where the grid
 // is small enough (two thirds of the SMs) not to share L2 bandwidth.  Two CTAs fit an SM, but clusters of more
-// than two stop finding places on a third more CTAs than SMs.
-// fp32: one CTA fits an SM; among the plans whose clusters all find one (clusters of more than two: 85 % of the
-// SMs) the one whose CTA fetches the least, 64 or 48 KB per 32-wide step, a 128-wide tile's longer reduction counted as
-// another 128 KB.
-// From six row tiles on a third more CTAs than run at once is taken, if their share of K is long (12 or, fp32, 24
-// steps): a batch has
-// padding, and the tiles it leaves empty cost next to nothing.
-SplitPlan gemm_split_plan(int max_m, int n, int k, bool tf32) {
+// than two stop finding places on a third more CTAs than SMs, and a short K does not pay for more either.
+// The projection in front of the attention gains least: up to one row tile only, and without a cluster where its
+// tiles leave three quarters of the SMs to the kernels around it.
+// fp32: one CTA fits an SM; among the plans whose clusters all find one the one whose CTA fetches the least, 64
+// or 48 KB per 32-wide step, a 128-wide tile's longer reduction counted as another 128 KB.  From six row tiles on a
+// third more CTAs than SMs is taken where K is long: a batch has padding, and the tiles it leaves empty cost next
+// to nothing (N = 768, K = 3072, capacity 1024: 1591 against 1727; full, the launch alone 44 us against 54).
+SplitPlan gemm_split_plan(int max_m, int n, int k, bool tf32, bool feeds_attention) {
   SplitPlan best;
   if (max_m <= 0) return best;
   const int num_kb = (k + (tf32 ? 31 : 63)) / (tf32 ? 32 : 64);
   const long long m_tiles = (max_m + BM - 1) / BM, sms = sm_count();
-  const bool padded = m_tiles >= 6;
+  constexpr int kCounts[] = {8, 6, 5, 4, 3, 2};
   if (!tf32) {
     const long long tiles = m_tiles * (n / 64);
-    if (n % 64 != 0) return best;
-    for (int splits = kMaxSplits; splits >= 1 && best.splits == 0; splits >>= 1) {
+    if (n % 64 != 0 || (feeds_attention && m_tiles > 1)) return best;
+    if (feeds_attention && num_kb <= 12 && 8 * tiles > sms && 4 * tiles <= sms) {
+      best.splits = 1;
+      return best;
+    }
+    for (const int splits : kCounts) {
       const int share = num_kb / splits;
       const long long ctas = tiles * splits;
-      if (share < 1 || (splits > 1 && (share < 3 || (share < 6 && 3 * ctas > 2 * sms)))) continue;
-      if (splits > 2 ? 3 * ctas <= 4 * sms
-                     : ctas <= 2 * sms || (splits == 2 && padded && share >= 12 && 3 * ctas <= 8 * sms))
-        best.splits = splits;
+      if (share < 3 || (share < 5 && 3 * ctas > 2 * sms)) continue;
+      if (splits == 2 && share >= 12 ? ctas > 2 * sms : 3 * ctas > 4 * sms) continue;
+      best.splits = splits;
+      return best;
     }
     return best;
   }
-  constexpr int kCounts[] = {2, 3, 4, 5, 6, 8};
+  const bool padded = m_tiles >= 6;
   for (const bool second_try : {false, true}) {
     int least = 0;
     for (const int bn : {64, 128}) {
@@ -576,8 +583,13 @@ SplitPlan gemm_split_plan(int max_m, int n, int k, bool tf32) {
         const int most = bn == 64 ? Cfg<true, 64>::kBlocks * Cfg<true, 64>::kUnitKb
                                   : Cfg<true, 128>::kBlocks * Cfg<true, 128>::kUnitKb;  // what TMEM holds
         if (num_kb / splits < 3 || share > most) continue;
-        if (second_try ? !(padded && share >= 24 && 3 * ctas <= 4 * sms) : 20 * ctas > (splits > 2 ? 17 : 20) * sms)
-          continue;
+        if (second_try) {
+          if (!(padded && share >= 24 && 3 * ctas <= 4 * sms)) continue;
+        } else {
+          // percent of the SMs the clusters of this size can count on
+          const int places = splits > 5 ? 66 : splits > 2 ? 88 : bn == 128 ? (padded ? 0 : 66) : 100;
+          if (100 * ctas > places * sms) continue;
+        }
         const int fetched = bn == 64 ? share * 48 : share * 64 + 128;
         if (best.splits == 0 || fetched < least) best.bn = bn, best.splits = splits, least = fetched;
       }

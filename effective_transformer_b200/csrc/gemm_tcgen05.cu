@@ -1361,7 +1361,9 @@ cudaError_t launch_gemm_tcgen05(const __half* a, const __half* w_packed, const _
     }
     lnp = *ln;
   }
-  if (const SplitPlan plan = has_ln(epilogue) ? SplitPlan() : gemm_split_plan(max_m, n, k, false); plan.splits != 0) {
+  // the QKV projection is the one without activation or residual behind its bias
+  const bool feeds_attention = epilogue == kEpiBias || epilogue == kEpiNormIn;
+  if (const SplitPlan plan = has_ln(epilogue) ? SplitPlan() : gemm_split_plan(max_m, n, k, false, feeds_attention); plan.splits != 0) {
     SplitGemm g;
     g.a = a, g.w = w_packed, g.bias = bias, g.residual = residual, g.c = c;
     g.m_ptr = m_ptr, g.max_m = max_m, g.n = n, g.k = k;
