@@ -379,6 +379,11 @@ cudaError_t launch_attention_tcgen05_long(const __half* q, const __half* k, cons
 size_t attention_plan_ints(int batch, int max_tokens);
 cudaError_t launch_attention_plan(const int* cu_seqlens, int batch, int max_tokens, int* plan,
                                   cudaStream_t stream);
+// The same from the packed rows' sequence numbers; also writes cu_seqlens (as
+// launch_seq_bounds_from_batch_idx does).
+bool attention_plan_from_rows_supported(int batch, int max_tokens);
+cudaError_t launch_attention_plan_from_rows(const int* batch_idx, const int* t_ptr, int batch, int max_tokens,
+                                            int* cu_seqlens, int* plan, cudaStream_t stream);
 cudaError_t launch_attention_tcgen05(const __half* q, const __half* k, const __half* v,
                                      long long token_stride, long long head_stride, __half* ctx,
                                      const int* plan, int batch, int max_tokens, int heads, int d,

@@ -1275,9 +1275,16 @@ int et_layer(et_handle_t h, int layer, const et_encoder_param_t* p, const et_tra
   }
   if (!h->layers[layer].ready) return set_error(h, ET_NOT_READY, "weights of this layer were never set");
   const int batch = tp->batch_size, seq = tp->from_seq_len, max_m = batch * seq;
-  ET_LAUNCH(h, ET_PROF_PADDING_OFFSETS, 1, s, launch_seq_bounds_from_batch_idx(p->batch_idx, p->valid_word_num, batch, max_m,
-                                              h->ws.cu_seqlens, s));
-  if (h->cfg.dtype == ET_FP16 && !h->use_simt && seq <= 128 && max_m > 0) {
+  const bool tiles = h->cfg.dtype == ET_FP16 && !h->use_simt && seq <= 128 && max_m > 0;
+  const bool one_kernel = tiles && batch > 0 && attention_plan_from_rows_supported(batch, max_m);
+  if (!one_kernel)
+    ET_LAUNCH(h, ET_PROF_PADDING_OFFSETS, 1, s, launch_seq_bounds_from_batch_idx(p->batch_idx, p->valid_word_num, batch, max_m,
+                                                h->ws.cu_seqlens, s));
+  if (one_kernel) {
+    ET_LAUNCH(h, ET_PROF_PADDING_OFFSETS, 1, s,
+              launch_attention_plan_from_rows(p->batch_idx, p->valid_word_num, batch, max_m, h->ws.cu_seqlens,
+                                              h->ws.attn_plan, s));
+  } else if (tiles) {
     ET_LAUNCH(h, ET_PROF_PADDING_OFFSETS, 1, s,
               launch_attention_plan(h->ws.cu_seqlens, batch, max_m, h->ws.attn_plan, s));
   } else if (h->cur_attr_mask != nullptr) {

@@ -569,3 +569,26 @@ def test_handles_on_two_devices_of_one_process():
             assert eng.device_status() == 0
             assert_parity(y, ref, sub.mask, fp16=True)
             eng.close()
+
+
+@pytest.mark.parametrize("lens", [[1], [0, 0, 5, 0, 128, 127, 1, 0], [128] * 5, [3, 0] * 200, [2] * 8128, [1] * 8129,
+                                  [100, 64, 33] * 50], ids=lambda v: f"{len(v)}_sequences")
+def test_layer_op_boundaries_from_row_indices(lens):
+    """The layer op has no sequence boundaries: one kernel works them out from batch_idx and plans the attention's
+    tiles (up to 16 384 positions and 8 128 sequences, two kernels beyond).  Same rows as the whole-stack call, which
+    plans from the boundaries of the input op; empty sequences at both ends, and both sides of the limits."""
+    batch, seq = len(lens), max(max(lens), 1)
+    spec = W.tiny_spec(dtype="fp16", batch=4)
+    sh = spec.shape
+    wl = W.make_workload(spec, random_gamma_beta=True)
+    eng = et.EffectiveTransformer(sh.num_layers, sh.head_num, sh.size_per_head, sh.ffn_dim, batch, seq,
+                                  dtype=torch.float16)
+    eng.set_weights(wl.weights)
+    gen = torch.Generator(device="cuda").manual_seed(batch + seq)
+    x = torch.randn(batch, seq, sh.hidden, device="cuda", dtype=torch.float16, generator=gen)
+    m = torch.from_numpy((np.arange(seq)[None] < np.asarray(lens)[:, None]).astype(np.int32)).cuda()
+    cfg = et.BertConfig(sh.hidden, sh.num_layers, sh.head_num, sh.ffn_dim)
+    whole = eng.forward(x, m)
+    ops = et.get_sequence_output(cfg, batch, seq, None, m, x, wl.weights, engine=eng)
+    assert torch.equal(whole, ops)
+    eng.close()
