@@ -150,10 +150,10 @@ __device__ __forceinline__ void weighted_values(const float (*Ps)[kPad], const f
 // for the CTA).
 template <typename T, bool kVec>
 __global__ void __launch_bounds__(kThreads, 4)
-attention_simt_kernel(const T* __restrict__ q, const T* __restrict__ k, const T* __restrict__ v,
+attention_simt_kernel(const T* q, const T* k, const T* v,
                       long long token_stride, long long head_stride, T* __restrict__ ctx, T* __restrict__ ctx_lo,
-                      const int* __restrict__ cu_seqlens, int heads, int max_seq, float scale,
-                      const int* __restrict__ cu_seqlens_k, long long kv_token_stride, int max_seq_k) {
+                      const int* cu_seqlens, int heads, int max_seq, float scale,
+                      const int* cu_seqlens_k, long long kv_token_stride, int max_seq_k) {
   pdl_wait();
   pdl_trigger();
   const int b = blockIdx.x / heads, head = blockIdx.x % heads;

@@ -106,8 +106,8 @@ __host__ __device__ inline size_t plan_ints(int batch, int max_tokens) {
 // dependent reads.
 // The op-by-op pass of the 100 x 32 batch, 12 layers: 1057 -> 1030 us with one kernel in place of two.
 constexpr int kSharedSeqs = 8128;
-__global__ void attention_plan_kernel(const int* __restrict__ cu_seqlens, const int* __restrict__ batch_idx,
-                                      const int* __restrict__ t_ptr, int* __restrict__ cu_out, int batch,
+__global__ void attention_plan_kernel(const int* cu_seqlens, const int* batch_idx,
+                                      const int* t_ptr, int* __restrict__ cu_out, int batch,
                                       int max_tokens, int* __restrict__ plan) {
   pdl_wait();
   pdl_trigger();
@@ -234,8 +234,8 @@ struct MaskArgs {
 // every head of every layer.
 constexpr int kMaskBitsStride = 8;
 __global__ void __launch_bounds__(256)
-mask_bits_kernel(const __half* __restrict__ attr_mask, const int* __restrict__ batch_idx,
-                 const int* __restrict__ word_idx, const int* __restrict__ cu_seqlens, const int* __restrict__ t_ptr,
+mask_bits_kernel(const __half* attr_mask, const int* batch_idx,
+                 const int* word_idx, const int* cu_seqlens, const int* t_ptr,
                  int max_tokens, int seq, uint32_t* __restrict__ out) {
   pdl_wait();
   pdl_trigger();
@@ -270,7 +270,7 @@ template <bool kMask>
 __global__ void __launch_bounds__(kThreads, kCtasPerSm)
 attention_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_k,
                          const __grid_constant__ CUtensorMap tmap_v, Coords co, __half* __restrict__ ctx,
-                         const int* __restrict__ plan, int batch, int max_tokens, int heads,
+                         const int* plan, int batch, int max_tokens, int heads,
                          float scale_log2e, int* status_word, int reverse, MaskArgs ma) {
   // The prologue (barriers, TMEM) touches no global memory: it runs before the
   // wait on the preceding kernel, under that kernel's tail.
@@ -623,7 +623,7 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_q, const __gri
 __global__ void __launch_bounds__(kThreads, kCtasPerSm)
 attention_tcgen05_long_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_k,
                               const __grid_constant__ CUtensorMap tmap_v, Coords co, __half* __restrict__ ctx,
-                              const int* __restrict__ cu_seqlens, int max_tokens, int max_seq, int heads, int q_tiles,
+                              const int* cu_seqlens, int max_tokens, int max_seq, int heads, int q_tiles,
                               float scale_log2e, int* status_word) {
   pdl_trigger();
   extern __shared__ __align__(1024) uint8_t smem_raw[];

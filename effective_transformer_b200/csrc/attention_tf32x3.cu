@@ -51,9 +51,9 @@ __device__ __forceinline__ void mma_3x(float (&c)[4], const uint32_t (&ah)[4], c
 
 template <bool kVec>
 __global__ void __launch_bounds__(kThreads, 4)
-attention_tf32x3_kernel(const float* __restrict__ q, const float* __restrict__ k, const float* __restrict__ v,
+attention_tf32x3_kernel(const float* q, const float* k, const float* v,
                         long long token_stride, long long head_stride, float* __restrict__ ctx,
-                        float* __restrict__ ctx_lo, const int* __restrict__ cu_seqlens, int heads, int max_seq,
+                        float* __restrict__ ctx_lo, const int* cu_seqlens, int heads, int max_seq,
                         float scale) {
   pdl_wait();
   pdl_trigger();

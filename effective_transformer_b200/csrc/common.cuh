@@ -75,7 +75,15 @@ class PerDeviceOnce {
 //     to global memory and before any exit path (it returns once the previous
 //     kernel has completed and its writes are visible);
 //   * pdl_trigger() only lets the next kernel start being scheduled earlier; it
-//     carries no ordering.
+//     carries no ordering;
+//   * what an earlier kernel of the stream may write -- activations, row statistics, the token
+//     count, sequence bounds, row indices, the attention plan -- is read by coherent loads.
+//     ld.global.nc is defined only for data that nobody writes while the kernel lives, and a
+//     CTA of such a kernel is alive (waiting) while its predecessors still store.  So those
+//     pointers carry no __restrict__ (const T* __restrict__ lets the compiler choose .nc, and
+//     move the load in front of the wait), and vectors of them come through
+//     ld_activation_v4().  Weights, biases, gamma, beta, column sums and embedding tables are
+//     complete before a pass begins and may keep both.
 // Without the launch attribute both instructions are no-ops.
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
@@ -126,11 +134,21 @@ struct alignas(16) Vec16 {
   uint32_t x, y, z, w;
 };
 
+// Weights and other data that no kernel of a pass writes.
 __device__ __forceinline__ Vec16 ld_global_nc_v4(const void* p) {
   Vec16 v;
   asm volatile("ld.global.nc.L1::no_allocate.v4.u32 {%0,%1,%2,%3}, [%4];"
                : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
                : "l"(p));
+  return v;
+}
+// A vector that an earlier kernel of the stream wrote (see the contract of pdl_wait above).
+__device__ __forceinline__ Vec16 ld_activation_v4(const void* p) {
+  Vec16 v;
+  asm volatile("ld.global.L1::no_allocate.v4.u32 {%0,%1,%2,%3}, [%4];"
+               : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
+               : "l"(p)
+               : "memory");
   return v;
 }
 // Through L2 only: for rows that other CTAs of the same kernel have just written.

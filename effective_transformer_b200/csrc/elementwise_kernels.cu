@@ -102,9 +102,9 @@ add_bias_gelu_kernel(T* __restrict__ out, const T* __restrict__ bias, const int*
 // keeping them in registers raises the number of resident warps.
 template <typename T, int kVPL, int kRows, bool kHasInput>
 __global__ void __launch_bounds__(kThreads, (kVPL <= 4 ? 2 : 1))
-add_bias_input_layernorm_kernel(T* __restrict__ out, const T* __restrict__ input,
+add_bias_input_layernorm_kernel(T* __restrict__ out, const T* input,
                                 const T* __restrict__ bias, const T* __restrict__ gamma,
-                                const T* __restrict__ beta, const int* __restrict__ t_ptr,
+                                const T* __restrict__ beta, const int* t_ptr,
                                 int max_tokens, int n, float eps, int reverse, T* __restrict__ split_hi,
                                 T* __restrict__ split_lo) {
   pdl_wait();
@@ -131,7 +131,7 @@ add_bias_input_layernorm_kernel(T* __restrict__ out, const T* __restrict__ input
           const int c = j * 32 + lane;
           if (c < vpr) {
             vo[k][j] = ld_global_v4(orow + c * E);
-            if (kHasInput) vi[k][j] = ld_global_nc_v4(input + static_cast<size_t>(rows[k]) * n + c * E);
+            if (kHasInput) vi[k][j] = ld_activation_v4(input + static_cast<size_t>(rows[k]) * n + c * E);
           }
         }
       }

@@ -110,7 +110,7 @@ struct Maps {
 template <bool kTf32, int BN, int EPI>
 __global__ void __launch_bounds__(kThreads, kTf32 ? 1 : 2)
 gemm_split_kernel(const __grid_constant__ Maps maps, void* __restrict__ c_ptr, float* __restrict__ c_lo,
-                  const void* __restrict__ bias_ptr, const void* __restrict__ res_ptr, const int* __restrict__ m_ptr,
+                  const void* __restrict__ bias_ptr, const void* res_ptr, const int* m_ptr,
                   int max_m, int N, int num_kb, int weights_ready, int* status_word, const GemmLayerNorm ln) {
   using cfg = Cfg<kTf32, BN>;
   using T = typename std::conditional<kTf32, float, __half>::type;
@@ -304,7 +304,7 @@ gemm_split_kernel(const __grid_constant__ Maps maps, void* __restrict__ c_ptr, f
 #pragma unroll
       for (int j = 0; j < 8; ++j)
         if (j < items && row_of(j) < rows) {
-          if constexpr (kResidual) res[j] = ld_global_nc_v4(residual + static_cast<size_t>(m0 + row_of(j)) * N + col);
+          if constexpr (kResidual) res[j] = ld_activation_v4(residual + static_cast<size_t>(m0 + row_of(j)) * N + col);
           if constexpr (is_deferred_norm(EPI)) {
             st[j][0] = st[j][1] = make_float2(0.f, 0.f);
             if (ln.stats_in != nullptr) {

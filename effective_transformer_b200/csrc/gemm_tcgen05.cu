@@ -84,7 +84,7 @@ __device__ __forceinline__ void ln_rows(__half* c, const __half* residual, const
 #pragma unroll
       for (int j = 0; j < VPL; ++j) {
         vc[r][j] = ld_global_cg_v4(c + off[r] + j * 256);
-        if (ADD) vr[r][j] = ld_global_nc_v4(residual + off[r] + j * 256);
+        if (ADD) vr[r][j] = ld_activation_v4(residual + off[r] + j * 256);
       }
     }
 #pragma unroll
@@ -326,7 +326,7 @@ __device__ __forceinline__ void epilogue_warp_tile(uint32_t t_row, __half* ctile
 #pragma unroll
       for (int i = 0; i < 8; ++i) {
         const int rr = 4 * i + g;
-        if (rr < rows_valid) res[i] = ld_global_nc_v4(rtile + static_cast<size_t>(rr) * N + c * 64 + piece * 8);
+        if (rr < rows_valid) res[i] = ld_activation_v4(rtile + static_cast<size_t>(rr) * N + c * 64 + piece * 8);
       }
       // gamma, beta of this lane's eight columns as fp16 pairs (fetched before the accumulator
       // arrived)
@@ -373,7 +373,7 @@ __device__ __forceinline__ void epilogue_warp_tile(uint32_t t_row, __half* ctile
 #pragma unroll
       for (int i = 0; i < 8; ++i) {
         const int rr = 4 * i + (lane >> 3), piece = lane & 7;
-        if (rr < rows_valid) res[i] = ld_global_nc_v4(rtile + static_cast<size_t>(rr) * N + c * 64 + piece * 8);
+        if (rr < rows_valid) res[i] = ld_activation_v4(rtile + static_cast<size_t>(rr) * N + c * 64 + piece * 8);
       }
 #pragma unroll
       for (int i = 0; i < 8; ++i) {
@@ -415,8 +415,8 @@ template <int BN, int EPI>
 __global__ void __launch_bounds__(kNumThreads, 1)
 gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a,
                     const __grid_constant__ CUtensorMap tmap_b, __half* __restrict__ C,
-                    const __half* __restrict__ bias, const __half* __restrict__ residual,
-                    const int* __restrict__ m_ptr, int max_m, int N, int K, int* status_word, int reverse_m) {
+                    const __half* __restrict__ bias, const __half* residual,
+                    const int* m_ptr, int max_m, int N, int K, int* status_word, int reverse_m) {
   using cfg = Cfg<BN>;
   constexpr int S = cfg::kStages;
 
@@ -658,8 +658,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(threads_of(EPI), 1)
 gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap tmap_a,
                          const __grid_constant__ CUtensorMap tmap_b,
                          const __grid_constant__ CUtensorMap tmap_b_half, __half* __restrict__ C,
-                         const __half* __restrict__ bias, const __half* __restrict__ residual,
-                         const int* __restrict__ m_ptr, int max_m, int N, int K, int* status_word,
+                         const __half* __restrict__ bias, const __half* residual,
+                         const int* m_ptr, int max_m, int N, int K, int* status_word,
                          int reverse_m, const GemmLayerNorm ln) {
   using cfg = PairCfg;
   constexpr int S = cfg::kStages;

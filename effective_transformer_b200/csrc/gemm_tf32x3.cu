@@ -187,7 +187,7 @@ __device__ __forceinline__ void store_chunk16(float* stage, const float* vals, f
 // may be the same array as x (each element is read, then written, by one thread).
 __global__ void __launch_bounds__(256)
 split_tf32_kernel(const float* x, float* hi, float* lo,
-                  const int* __restrict__ rows_ptr, int max_rows, int cols) {
+                  const int* rows_ptr, int max_rows, int cols) {
   pdl_wait();
   pdl_trigger();
   int rows = rows_ptr != nullptr ? *rows_ptr : max_rows;
@@ -228,7 +228,7 @@ __global__ void __launch_bounds__(kNumThreads, 1)
 gemm_tf32x3_kernel(const __grid_constant__ CUtensorMap tmap_a_hi, const __grid_constant__ CUtensorMap tmap_a_lo,
                    const __grid_constant__ CUtensorMap tmap_w_hi, const __grid_constant__ CUtensorMap tmap_w_lo,
                    float* __restrict__ C, float* __restrict__ c_lo, const float* __restrict__ bias,
-                   const int* __restrict__ m_ptr, int max_m, int N, int K, int* status_word, int reverse_m) {
+                   const int* m_ptr, int max_m, int N, int K, int* status_word, int reverse_m) {
   using cfg = Cfg;
   constexpr int S = cfg::kStages;
 
@@ -491,7 +491,7 @@ gemm_tf32x3_pair_kernel(const __grid_constant__ CUtensorMap tmap_a_hi, const __g
                         const __grid_constant__ CUtensorMap tmap_w_hi, const __grid_constant__ CUtensorMap tmap_w_lo,
                         const __grid_constant__ CUtensorMap tmap_w_hi_half,
                         const __grid_constant__ CUtensorMap tmap_w_lo_half, float* __restrict__ C,
-                        float* __restrict__ c_lo, const float* __restrict__ bias, const int* __restrict__ m_ptr,
+                        float* __restrict__ c_lo, const float* __restrict__ bias, const int* m_ptr,
                         int max_m, int N, int K, int* status_word, int reverse_m) {
   using cfg = PairCfg;
   constexpr int S = cfg::kStages;

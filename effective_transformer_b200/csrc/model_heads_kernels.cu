@@ -28,9 +28,9 @@ __device__ __forceinline__ int clamp_tokens(const int* t_ptr, int max_tokens) {
 // TensorFlow's GPU gather and one-hot matmul do.
 template <typename T, int kVPL>
 __global__ void __launch_bounds__(kThreads, (kVPL <= 4 ? kCtasPerSm : 1))
-embedding_layernorm_kernel(const int* __restrict__ input_ids, const int* __restrict__ token_type_ids,
-                           const int* __restrict__ batch_idx, const int* __restrict__ word_idx,
-                           const int* __restrict__ t_ptr, const T* __restrict__ word_table, int vocab,
+embedding_layernorm_kernel(const int* input_ids, const int* token_type_ids,
+                           const int* batch_idx, const int* word_idx,
+                           const int* t_ptr, const T* __restrict__ word_table, int vocab,
                            const T* __restrict__ type_table, int type_vocab,
                            const T* __restrict__ pos_table, const T* __restrict__ gamma,
                            const T* __restrict__ beta, T* __restrict__ out, int max_tokens, int seq,
@@ -127,7 +127,7 @@ embedding_layernorm_kernel(const int* __restrict__ input_ids, const int* __restr
 // (may be null) receives the number of rows written, for a GEMM that reads
 // its row count from the device.
 __global__ void __launch_bounds__(kThreads)
-gather_first_tokens_kernel(const char* __restrict__ packed, const int* __restrict__ cu_seqlens,
+gather_first_tokens_kernel(const char* packed, const int* cu_seqlens,
                            char* __restrict__ out, int batch, int max_tokens, int row_bytes,
                            int* __restrict__ count_out) {
   pdl_wait();
@@ -145,7 +145,7 @@ gather_first_tokens_kernel(const char* __restrict__ packed, const int* __restric
     char* dst = out + static_cast<size_t>(b) * row_bytes;
     for (int i = lane; i < nvec; i += 32)
       st_global_v4(dst + static_cast<size_t>(i) * 16,
-                   has ? ld_global_nc_v4(src + static_cast<size_t>(i) * 16) : zero);
+                   has ? ld_activation_v4(src + static_cast<size_t>(i) * 16) : zero);
   }
 }
 

@@ -18,7 +18,7 @@ constexpr int kRowsPerCta = 8;  // one warp per mask row
 
 // Pass 1: valid positions per mask row.
 __global__ void __launch_bounds__(kRowsPerCta * 32)
-seq_lengths_kernel(const int* __restrict__ mask, int batch, int seq, int* __restrict__ lens,
+seq_lengths_kernel(const int* mask, int batch, int seq, int* __restrict__ lens,
                    int* __restrict__ seq_len_out) {
   pdl_wait();
   pdl_trigger();
@@ -38,7 +38,7 @@ seq_lengths_kernel(const int* __restrict__ mask, int batch, int seq, int* __rest
 
 // Pass 2: row bases from the row lengths, then a ballot scan inside each row.
 __global__ void __launch_bounds__(kRowsPerCta * 32)
-padding_offsets_emit_kernel(const int* __restrict__ mask, const int* __restrict__ lens, int batch,
+padding_offsets_emit_kernel(const int* mask, const int* lens, int batch,
                             int seq, int* __restrict__ prefix_sum, int* __restrict__ valid_word_num,
                             int* __restrict__ batch_idx, int* __restrict__ word_idx,
                             int* __restrict__ cu_seqlens, int* __restrict__ padding_offset) {
@@ -94,7 +94,7 @@ __global__ void empty_batch_kernel(int* valid_word_num, int* cu_seqlens) {
 
 // cu_seqlens from batch_idx alone (the layer op receives no other padding
 // information): packed rows of one sequence are contiguous and ordered by b.
-__global__ void seq_bounds_kernel(const int* __restrict__ batch_idx, const int* __restrict__ t_ptr,
+__global__ void seq_bounds_kernel(const int* batch_idx, const int* t_ptr,
                                   int batch, int max_tokens, int* __restrict__ cu_seqlens) {
   pdl_wait();
   pdl_trigger();
@@ -113,14 +113,14 @@ constexpr int kCopyWarpsPerCta = 8;
 constexpr int kCopyCtasPerSm = 8;
 
 template <int kChunk>
-__device__ __forceinline__ void warp_copy_row(const char* __restrict__ src, char* __restrict__ dst,
+__device__ __forceinline__ void warp_copy_row(const char* src, char* __restrict__ dst,
                                               int nvec, int lane) {
   for (int i0 = 0; i0 < nvec; i0 += 32 * kChunk) {
     Vec16 r[kChunk];
 #pragma unroll
     for (int c = 0; c < kChunk; ++c) {
       const int i = i0 + c * 32 + lane;
-      if (i < nvec) r[c] = ld_global_nc_v4(src + static_cast<size_t>(i) * 16);
+      if (i < nvec) r[c] = ld_activation_v4(src + static_cast<size_t>(i) * 16);
     }
 #pragma unroll
     for (int c = 0; c < kChunk; ++c) {
@@ -137,8 +137,8 @@ __device__ __forceinline__ void warp_zero_row(char* __restrict__ dst, int nvec, 
 
 // Packed row v <- padded row (batch_idx[v], word_idx[v]); one warp per row.
 __global__ void __launch_bounds__(kCopyWarpsPerCta * 32)
-remove_padding_kernel(const char* __restrict__ from, const int* __restrict__ batch_idx,
-                      const int* __restrict__ word_idx, const int* __restrict__ t_ptr,
+remove_padding_kernel(const char* from, const int* batch_idx,
+                      const int* word_idx, const int* t_ptr,
                       char* __restrict__ to, int max_rows, int seq, int row_bytes) {
   pdl_wait();
   pdl_trigger();
@@ -163,8 +163,8 @@ remove_padding_kernel(const char* __restrict__ from, const int* __restrict__ bat
 // item, the warp in front of a short sequence's padding filled all of it alone
 // (32 x 512 positions, gaps of up to 448 rows: 51.7 us under ncu for 39 MB).
 __global__ void __launch_bounds__(kCopyWarpsPerCta * 32)
-restore_padding_kernel(const char* __restrict__ from, const int* __restrict__ batch_idx,
-                       const int* __restrict__ word_idx, const int* __restrict__ t_ptr,
+restore_padding_kernel(const char* from, const int* batch_idx,
+                       const int* word_idx, const int* t_ptr,
                        char* __restrict__ to, int max_rows, int seq, int row_bytes) {
   constexpr int kItems = kCopyWarpsPerCta * 32;
   __shared__ int gap_lo[kItems], gap_hi[kItems];  // padded rows [lo, hi) in front of an item; hi = the item's own row

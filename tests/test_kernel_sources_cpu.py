@@ -1,0 +1,58 @@
+"""Rules that every kernel of a pass keeps, checked on its source.
+
+A kernel launched while its predecessors still run (programmatic dependent launch) may not read what they write
+through the non-coherent path: ld.global.nc, and const T* __restrict__, which lets the compiler choose it and move
+the load in front of griddepcontrol.wait.  No run shows such a load reliably, so the sources are read instead.
+"""
+import os
+import re
+
+import pytest
+
+CSRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "effective_transformer_b200", "csrc")
+FILES = sorted(f for f in os.listdir(CSRC) if f.endswith(".cu"))
+# complete before a pass begins: weights and what is worked out from them
+CONSTANT = {"bias", "bias_ptr", "gamma", "beta", "word_table", "type_table", "pos_table"}
+CONSTANT_VECTOR = re.compile(r"ld_global_nc_v4\((p\b|\(lane < 8 \? nc\.bias_g : nc\.csum_g\)|ln\.gamma|ln\.beta|wrow)")
+
+
+def kernels(text):
+    """(name, parameter list, body) of every __global__ function."""
+    for m in re.finditer(r"__global__", text):
+        name = re.compile(r"(\w+_kernel)\(").search(text, m.end())
+        depth, i = 1, name.end()
+        while depth:
+            depth += {"(": 1, ")": -1}.get(text[i], 0)
+            i += 1
+        params = text[name.end():i - 1]
+        start = text.index("{", i)
+        depth, j = 1, start + 1
+        while depth:
+            depth += {"{": 1, "}": -1}.get(text[j], 0)
+            j += 1
+        yield name.group(1), params, text[start:j]
+
+
+def read(name):
+    with open(os.path.join(CSRC, name)) as f:
+        return re.sub(r"//[^\n]*", "", f.read())
+
+
+def test_the_parser_sees_the_kernels():
+    names = [k for f in FILES for k, _, _ in kernels(read(f))]
+    assert {"gemm_split_kernel", "gemm_tcgen05_pair_kernel", "gemm_tf32x3_pair_kernel", "attention_tcgen05_kernel",
+            "attention_tcgen05_long_kernel", "restore_padding_kernel", "add_bias_input_layernorm_kernel"} <= set(names)
+
+
+@pytest.mark.parametrize("name", FILES)
+def test_what_an_earlier_kernel_writes_is_read_coherently(name):
+    for kernel, params, body in kernels(read(name)):
+        if "pdl_wait()" not in body:
+            continue  # launched in plain stream order
+        restrict = re.findall(r"const\s+[\w:]+\s*\*\s*__restrict__\s+(\w+)", params)
+        assert set(restrict) <= CONSTANT, f"{name}: {kernel}: {sorted(set(restrict) - CONSTANT)}"
+    text = read(name)
+    if "pdl_wait()" in text:
+        for call in re.findall(r"ld_global_nc_v4\([^;]*", text):
+            # (the standalone bias + transpose kernel is launched in plain stream order)
+            assert CONSTANT_VECTOR.match(call) or "srcs[w]" in call, f"{name}: {call}"
