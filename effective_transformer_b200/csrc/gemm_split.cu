@@ -211,6 +211,12 @@ gemm_split_kernel(const __grid_constant__ Maps maps, void* __restrict__ c_ptr, f
           load_a(kb0 + issued, s);
         }
       }
+      // the issuer's commits on the empty barriers are asynchronous arrivals: the last of them land before the
+      // barriers go away
+      if (live)
+        for (int i = max(0, issued - S); i < issued; ++i)
+          if (!mbar_wait(empty_bar(i % S), static_cast<uint32_t>((i / S) & 1), abort_flag) && *abort_flag == 0)
+            fail(kSiteDrain);
       // copies in flight must land before the CTA's shared memory goes away
       for (int i = max(0, issued - S); i < issued; ++i)
         if (!mbar_wait(full_bar(i % S), static_cast<uint32_t>((i / S) & 1), abort_flag) && *abort_flag == 0)

@@ -325,6 +325,14 @@ gemm_tf32x3_kernel(const __grid_constant__ CUtensorMap tmap_a_hi, const __grid_c
           }
         }
       }
+      // the issuer's commits on empty[] are asynchronous arrivals: the last of them land before the barriers go away
+      const long long unread = issued < S ? issued : S;
+      for (long long i = 0; i < unread; ++i) {
+        const long long f = issued - 1 - i;
+        if (!mbar_wait(empty_bar(static_cast<int>(f % S)), static_cast<uint32_t>((f / S) & 1), abort_flag) &&
+            *abort_flag == 0)
+          fail(kSiteProducerDrain);
+      }
       // copies still in flight must land before the CTA's shared memory goes away
       const long long pending = issued < S ? issued : S;
       for (long long i = 0; i < pending; ++i) {
@@ -596,6 +604,16 @@ gemm_tf32x3_pair_kernel(const __grid_constant__ CUtensorMap tmap_a_hi, const __g
             phase ^= 1u;
           }
         }
+      }
+      // The issuer's commits arrive on this CTA's empty[] barriers asynchronously, in the peer from the
+      // other SM, and nothing else waits for the last of them: an arrival must not find the barrier's
+      // memory given to another CTA.
+      const long long unread = issued < S ? issued : S;
+      for (long long i = 0; i < unread; ++i) {
+        const long long f = issued - 1 - i;
+        if (!mbar_wait(empty_bar(static_cast<int>(f % S)), static_cast<uint32_t>((f / S) & 1), abort_flag) &&
+            *abort_flag == 0)
+          fail(kSiteProducerDrain);
       }
       if (rank == 0) {
         // full[] counts both CTAs' bytes: once these phases are complete no copy

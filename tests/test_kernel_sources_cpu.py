@@ -56,3 +56,16 @@ def test_what_an_earlier_kernel_writes_is_read_coherently(name):
         for call in re.findall(r"ld_global_nc_v4\([^;]*", text):
             # (the standalone bias + transpose kernel is launched in plain stream order)
             assert CONSTANT_VECTOR.match(call) or "srcs[w]" in call, f"{name}: {call}"
+
+
+def test_ring_commits_are_waited_for_before_the_barriers_go_away():
+    """tcgen05.commit arrives on a barrier asynchronously, in the CTA-pair kernels on the peer's.  A kernel that frees
+    its ring with such arrivals outstanding could have them land in another CTA's shared memory: the producer waits
+    for its stages once inside the loop and once behind it."""
+    seen = 0
+    for name in FILES:
+        for kernel, _, body in kernels(read(name)):
+            if re.search(r"umma_commit(_pair)?\(empty_bar", body):
+                seen += 1
+                assert body.count("mbar_wait(empty_bar(") == 2, f"{name}: {kernel}"
+    assert seen == 5
