@@ -423,7 +423,8 @@ cudaError_t launch_split_tf32(const float* x, float* hi, float* lo, const int* r
 cudaError_t launch_gemm_tf32x3(const float* a_hi, const float* a_lo, const float* w_hi, const float* w_lo,
                                const float* bias, float* c, const int* m_ptr, int max_m, int n, int k,
                                int epilogue, int* status_word, cudaStream_t stream, bool reverse_m = false,
-                               float* c_lo = nullptr, TensorMapCache* maps = nullptr, bool weights_ready = false);
+                               float* c_lo = nullptr, TensorMapCache* maps = nullptr, bool weights_ready = false,
+                               int route_rows = 0);
 // tcgen05 GEMM, fp16 in / fp32 accumulate / fp16 out.  w_packed is [N,K].
 // reverse_m: row tiles are visited from the last to the first.  A kernel that
 // consumes what the previous kernel has just written finds the rows written
@@ -431,11 +432,13 @@ cudaError_t launch_gemm_tf32x3(const float* a_hi, const float* a_lo, const float
 // alternate their direction.
 // weights_ready: w_packed was complete before the preceding kernel of the stream began (the handle's own
 // weights), so a kernel may fetch it before it waits for that kernel.
+// route_rows: the capacity in rows by which the kernel is chosen, 0 = max_m.  The kernels round differently (order
+// of the K sum, fp16 pairs or fp32 in an epilogue), so the parts of one batch name the whole batch's here.
 cudaError_t launch_gemm_tcgen05(const __half* a, const __half* w_packed, const __half* bias,
                                 __half* c, const int* m_ptr, int max_m, int n, int k, int epilogue,
                                 int* status_word, cudaStream_t stream, bool reverse_m = false,
                                 const __half* residual = nullptr, TensorMapCache* maps = nullptr,
-                                const GemmLayerNorm* ln = nullptr, bool weights_ready = false);
+                                const GemmLayerNorm* ln = nullptr, bool weights_ready = false, int route_rows = 0);
 // Projections of small batches on tiles of 128 x 64 (fp32 also 128 x 128) whose K range is split over a cluster
 // (gemm_split.cu).  fp16: a [max_m,k], w [n,k], c fp16.  a_lo / w_lo given: fp32 by the three-product tf32
 // split, c_lo as in launch_gemm_tf32x3.

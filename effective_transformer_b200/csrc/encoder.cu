@@ -217,6 +217,9 @@ struct et_handle_s {
   const int* cur_word_idx = nullptr;
   const int* cur_batch_idx = nullptr;
   bool mask_bits_ready = false;  // ws.mask_bits holds that mask (inside a whole-stack call)
+  // Rows by which the projections' kernels are chosen, 0 = the pass's own capacity.  A host-buffer call sets the
+  // whole batch's for the passes over its chunks: their shares follow measured times, the result must not.
+  int route_rows = 0;
   std::vector<LayerWeights> layers;
   ModelWeights model;
   Workspace ws;
@@ -346,6 +349,12 @@ struct MaskScope {
   }
 };
 
+struct RouteScope {
+  et_handle_t h;
+  RouteScope(et_handle_t handle, int rows) : h(handle) { h->route_rows = rows; }
+  ~RouteScope() { h->route_rows = 0; }
+};
+
 int ws_alloc(et_handle_t h, void** p, size_t bytes) {
   bytes = ws_round(bytes);
   ET_CUDA(h, cudaMalloc(p, bytes));
@@ -461,7 +470,8 @@ int run_layer(et_handle_t h, const LayerWeights& lw, const T* x_in, T* x_out, co
     if (tc)
       return launch_gemm_tcgen05(reinterpret_cast<const __half*>(a), static_cast<const __half*>(w_t),
                                  static_cast<const __half*>(bias), reinterpret_cast<__half*>(c), t_ptr,
-                                 max_m, n, k, epi, ws.status, s, turn(), nullptr, &h->maps, nullptr, true);
+                                 max_m, n, k, epi, ws.status, s, turn(), nullptr, &h->maps, nullptr, true,
+                                 h->route_rows);
     if (tc32) {
       // w_t holds rn_tf32(W), w_lo the remainder; the input is split the same way first
       const float* a_hi = reinterpret_cast<const float*>(a);
@@ -474,7 +484,7 @@ int run_layer(et_handle_t h, const LayerWeights& lw, const T* x_in, T* x_out, co
       }
       return launch_gemm_tf32x3(a_hi, a_lo, static_cast<const float*>(w_t), static_cast<const float*>(w_lo),
                                 static_cast<const float*>(bias), reinterpret_cast<float*>(c), t_ptr, max_m, n, k,
-                                epi, ws.status, s, turn(), c_lo, &h->maps, true);
+                                epi, ws.status, s, turn(), c_lo, &h->maps, true, h->route_rows);
     }
     forward_only();
     return launch_gemm_simt<T>(a, B(w_rm), B(bias), c, t_ptr, max_m, n, k, epi, s);
@@ -497,7 +507,8 @@ int run_layer(et_handle_t h, const LayerWeights& lw, const T* x_in, T* x_out, co
     nin.csum = H16(lw.cqkv);
     ET_LAUNCH(h, ET_PROF_GEMM_QKV, 1, s,
               launch_gemm_tcgen05(H16(x_in), H16(lw.wqkv_f), H16(lw.bqkv_f), reinterpret_cast<__half*>(qkv), t_ptr,
-                                  max_m, 3 * hid, hid, kEpiNormIn, ws.status, s, turn(), nullptr, &h->maps, &nin, true));
+                                  max_m, 3 * hid, hid, kEpiNormIn, ws.status, s, turn(), nullptr, &h->maps, &nin, true,
+                                  h->route_rows));
   } else if (tc32 && in_split_ready)
     ET_LAUNCH(h, ET_PROF_GEMM_QKV, 1, s,
               gemm(reinterpret_cast<const T*>(ws.a_hi), lw.wqkv, lw.wqkv_t, lw.wqkv_lo, lw.bqkv, qkv, 3 * hid, hid,
@@ -562,7 +573,8 @@ int run_layer(et_handle_t h, const LayerWeights& lw, const T* x_in, T* x_out, co
     n1.stats_out = ws.stats_att;
     ET_LAUNCH(h, ET_PROF_GEMM_ATTN_OUT, 1, s,
               launch_gemm_tcgen05(H16(ctx), H16(lw.wo_t), H16(lw.bo), reinterpret_cast<__half*>(att), t_ptr, max_m,
-                                  hid, hid, kEpiNormResidual, ws.status, s, turn(), H16(x_in), &h->maps, &n1, true));
+                                  hid, hid, kEpiNormResidual, ws.status, s, turn(), H16(x_in), &h->maps, &n1, true,
+                                  h->route_rows));
     // first feed-forward projection of LN1(att): folded weights, statistics, GELU
     GemmLayerNorm n2;
     n2.eps = h->eps;
@@ -571,7 +583,7 @@ int run_layer(et_handle_t h, const LayerWeights& lw, const T* x_in, T* x_out, co
     n2.csum = H16(lw.c1);
     ET_LAUNCH(h, ET_PROF_GEMM_FFN1, 1, s,
               launch_gemm_tcgen05(H16(att), H16(lw.w1_f), H16(lw.b1_f), reinterpret_cast<__half*>(ffn), t_ptr, max_m,
-                                  f, hid, kEpiNormInGelu, ws.status, s, turn(), nullptr, &h->maps, &n2, true));
+                                  f, hid, kEpiNormInGelu, ws.status, s, turn(), nullptr, &h->maps, &n2, true, h->route_rows));
     // second: + bias + LN1(att) on the fly; leaves the sum in x_out and its statistics in ws.stats_x
     GemmLayerNorm n3;
     n3.eps = h->eps;
@@ -582,7 +594,7 @@ int run_layer(et_handle_t h, const LayerWeights& lw, const T* x_in, T* x_out, co
     n3.stats_out = ws.stats_x;
     ET_LAUNCH(h, ET_PROF_GEMM_FFN2, 1, s,
               launch_gemm_tcgen05(H16(ffn), H16(lw.w2_t), H16(lw.b2), reinterpret_cast<__half*>(x_out), t_ptr, max_m,
-                                  hid, f, kEpiNormResidual, ws.status, s, turn(), H16(att), &h->maps, &n3, true));
+                                  hid, f, kEpiNormResidual, ws.status, s, turn(), H16(att), &h->maps, &n3, true, h->route_rows));
     return ET_OK;
   }
   const bool ln_in_gemm = tc && h->fuse_ln && gemm_layernorm_supported(hid);
@@ -625,7 +637,8 @@ int run_layer(et_handle_t h, const LayerWeights& lw, const T* x_in, T* x_out, co
   } else if (tc) {
     ET_LAUNCH(h, ET_PROF_GEMM_FFN2, 1, s,
               launch_gemm_tcgen05(H16(ffn), H16(lw.w2_t), H16(lw.b2), reinterpret_cast<__half*>(x_out), t_ptr, max_m,
-                                  hid, f, kEpiBiasResidual, ws.status, s, turn(), H16(att), &h->maps, nullptr, true));
+                                  hid, f, kEpiBiasResidual, ws.status, s, turn(), H16(att), &h->maps, nullptr, true,
+                                  h->route_rows));
     ET_LAUNCH(h, ET_PROF_LAYERNORM, 1, s,
               launch_add_bias_input_layernorm<T>(x_out, nullptr, nullptr, B(lw.ln2_gamma), B(lw.ln2_beta), t_ptr,
                                                  max_m, hid, h->eps, s, turn()));
@@ -1368,6 +1381,7 @@ int forward_host_body(et_handle_t h, const void* from_host, const int* mask_host
   // when its upload has landed, and its result goes back on the download
   // stream while chunk i+1 is being computed.
   const size_t seq_bytes = static_cast<size_t>(seq_len) * h->hidden * h->esize;
+  const RouteScope route(h, batch_size * seq_len);
   int chunks = h->host_chunks;
   if (h->host_share_auto && h->host_share_measured && (h->tuned_batch != batch_size || h->tuned_seq != seq_len)) {
     h->host_share_measured = false;  // another shape: measure again, starting from the default shares

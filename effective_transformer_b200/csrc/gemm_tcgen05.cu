@@ -1340,7 +1340,7 @@ bool encode_2d_fp16_sw128(CUtensorMap* map, const void* base, uint64_t rows, uin
 cudaError_t launch_gemm_tcgen05(const __half* a, const __half* w_packed, const __half* bias,
                                 __half* c, const int* m_ptr, int max_m, int n, int k, int epilogue,
                                 int* status_word, cudaStream_t stream, bool reverse_m, const __half* residual,
-                                TensorMapCache* maps, const GemmLayerNorm* ln, bool weights_ready) {
+                                TensorMapCache* maps, const GemmLayerNorm* ln, bool weights_ready, int route_rows) {
   if (max_m <= 0) return cudaSuccess;
   if (n <= 0 || k <= 0 || (n % 128) != 0 || (k % 8) != 0) return cudaErrorInvalidValue;
   if ((reinterpret_cast<uintptr_t>(a) & 15u) || (reinterpret_cast<uintptr_t>(w_packed) & 15u) ||
@@ -1381,7 +1381,9 @@ cudaError_t launch_gemm_tcgen05(const __half* a, const __half* w_packed, const _
   }
   // the QKV projection is the one without activation or residual behind its bias
   const bool feeds_attention = epilogue == kEpiBias || epilogue == kEpiNormIn;
-  if (const SplitPlan plan = has_ln(epilogue) ? SplitPlan() : gemm_split_plan(max_m, n, k, false, feeds_attention); plan.splits != 0) {
+  if (route_rows <= 0) route_rows = max_m;
+  if (const SplitPlan plan = has_ln(epilogue) ? SplitPlan() : gemm_split_plan(route_rows, n, k, false, feeds_attention);
+      plan.splits != 0) {
     SplitGemm g;
     g.a = a, g.w = w_packed, g.bias = bias, g.residual = residual, g.c = c;
     g.m_ptr = m_ptr, g.max_m = max_m, g.n = n, g.k = k;
