@@ -415,27 +415,53 @@ int pack_layer_any(et_handle_t h, int layer, const void* const* w, cudaStream_t 
   return h->cfg.dtype == ET_FP16 ? pack_layer<__half>(h, lw, w, s) : pack_layer<float>(h, lw, w, s);
 }
 
+inline const __half* as_half(const void* p) { return static_cast<const __half*>(p); }
+inline __half* as_half(void* p) { return static_cast<__half*>(p); }
+
+// LN1 of layer l folded into its first feed-forward projection.
+int fold_ffn1(et_handle_t h, size_t l, cudaStream_t s) {
+  LayerWeights& lw = h->layers[l];
+  ET_CUDA(h, launch_fold_layernorm(as_half(lw.w1_t), as_half(lw.b1), as_half(lw.ln1_gamma), as_half(lw.ln1_beta),
+                                   as_half(lw.w1_f), as_half(lw.c1), as_half(lw.b1_f), h->cfg.ffn_dim, h->hidden, s));
+  return ET_OK;
+}
+// LN2 of layer l - 1 folded into layer l's QKV projection (the first layer's input is not normalised).
+int fold_qkv(et_handle_t h, size_t l, cudaStream_t s) {
+  if (l == 0 || l >= h->layers.size()) return ET_OK;
+  LayerWeights& lw = h->layers[l];
+  const LayerWeights& prev = h->layers[l - 1];
+  ET_CUDA(h, launch_fold_layernorm(as_half(lw.wqkv_t), as_half(lw.bqkv), as_half(prev.ln2_gamma),
+                                   as_half(prev.ln2_beta), as_half(lw.wqkv_f), as_half(lw.cqkv), as_half(lw.bqkv_f),
+                                   3 * h->hidden, h->hidden, s));
+  return ET_OK;
+}
+
 // Folded weights of every layer (deferred LayerNorm), once all layers have their weights.
 int fold_all(et_handle_t h, cudaStream_t s) {
   h->folded_ready = false;
   if (!defer_eligible(h->cfg)) return ET_OK;
   for (const auto& lw : h->layers)
     if (!lw.ready) return ET_OK;
-  const int hid = h->hidden, f = h->cfg.ffn_dim;
-  auto H16 = [](const void* p) { return static_cast<const __half*>(p); };
-  auto M16 = [](void* p) { return static_cast<__half*>(p); };
   for (size_t l = 0; l < h->layers.size(); ++l) {
-    LayerWeights& lw = h->layers[l];
-    ET_CUDA(h, launch_fold_layernorm(H16(lw.w1_t), H16(lw.b1), H16(lw.ln1_gamma), H16(lw.ln1_beta), M16(lw.w1_f),
-                                     M16(lw.c1), M16(lw.b1_f), f, hid, s));
-    if (l > 0) {
-      const LayerWeights& prev = h->layers[l - 1];
-      ET_CUDA(h, launch_fold_layernorm(H16(lw.wqkv_t), H16(lw.bqkv), H16(prev.ln2_gamma), H16(prev.ln2_beta),
-                                       M16(lw.wqkv_f), M16(lw.cqkv), M16(lw.bqkv_f), 3 * hid, hid, s));
-    }
+    int rc = fold_ffn1(h, l, s);
+    if (rc == ET_OK) rc = fold_qkv(h, l, s);
+    if (rc != ET_OK) return rc;
   }
   h->folded_ready = true;
   return ET_OK;
+}
+
+// Layer l's weights were replaced by the layer op: its own folded projections follow, and those of the next
+// layer's QKV projection, which hold its LN2.  In place and in stream order, as the packed weights themselves, so
+// that recorded passes see the new weights in both.
+int refold_layer(et_handle_t h, size_t l, cudaStream_t s) {
+  if (!h->folded_ready) return ET_OK;  // nothing uses folded weights until every layer has been set
+  h->folded_ready = false;             // should a launch fail: the passes run LayerNorm kernels
+  int rc = fold_ffn1(h, l, s);
+  if (rc == ET_OK) rc = fold_qkv(h, l, s);
+  if (rc == ET_OK) rc = fold_qkv(h, l + 1, s);
+  h->folded_ready = rc == ET_OK;
+  return rc;
 }
 
 // One encoder layer on the packed layout.  x_out may alias x_in.
@@ -1284,6 +1310,7 @@ int et_layer(et_handle_t h, int layer, const et_encoder_param_t* p, const et_tra
     for (int i = 0; i < 16; ++i)
       if (w[i] == nullptr) return set_error(h, ET_INVALID_ARGUMENT, "null weight pointer");
     rc = pack_layer_any(h, layer, w, s);
+    if (rc == ET_OK) rc = refold_layer(h, static_cast<size_t>(layer), s);
     if (rc != ET_OK) return rc;
   }
   if (!h->layers[layer].ready) return set_error(h, ET_NOT_READY, "weights of this layer were never set");

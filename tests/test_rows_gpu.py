@@ -3,11 +3,14 @@
 A mean over a batch hides one wrong row, and a wrong row of an early layer is diluted by the later ones; so the
 largest relative error of any row is taken, on batches whose contents change from call to call.
 """
+import ctypes as C
+
 import numpy as np
 import pytest
 import torch
 
 import effective_transformer_b200 as et
+from effective_transformer_b200 import _capi
 from effective_transformer_b200 import workloads as W
 
 pytestmark = pytest.mark.gpu
@@ -15,17 +18,23 @@ pytestmark = pytest.mark.gpu
 LARGE = dict(heads=16, ffn=4096)
 
 
+def make_weights(layers, h, ffn, seed=1):
+    """Sixteen tensors per layer, fp16 values whatever the handle; gamma around one, beta around zero."""
+    gen = torch.Generator(device="cuda").manual_seed(seed)
+
+    def normal(*shape):
+        return (0.02 * torch.randn(*shape, generator=gen, device="cuda")).half()
+
+    for _ in range(layers):
+        w = [normal(h, h) if i % 2 == 0 else normal(h) for i in range(8)]
+        yield w + [normal(h), 1 + 5 * normal(h), normal(h, ffn), normal(ffn), normal(ffn, h), normal(h), normal(h),
+                   1 + 5 * normal(h)]
+
+
 def make_engine(layers, batch, seq, heads, ffn, dtype=torch.float16, seed=1):
     h = heads * 64
     eng = et.EffectiveTransformer(layers, heads, 64, ffn, batch, seq, dtype=dtype)
-    gen = torch.Generator(device="cuda").manual_seed(seed)
-
-    def normal(*shape, scale=0.02):  # fp16 values in every handle
-        return (scale * torch.randn(*shape, generator=gen, device="cuda")).half()
-
-    for layer in range(layers):
-        w = [normal(h, h) if i % 2 == 0 else normal(h) for i in range(8)]
-        w += [normal(h), 1 + normal(h), normal(h, ffn), normal(ffn), normal(ffn, h), normal(h), normal(h), 1 + normal(h)]
+    for layer, w in enumerate(make_weights(layers, h, ffn, seed)):
         eng.set_layer_weights(layer, [t.to(dtype).cpu() for t in w])
     return eng
 
@@ -55,3 +64,56 @@ def test_host_call_rows_do_not_depend_on_the_chunk_shares(monkeypatch, dtype, se
             assert rows.size == 0, f"share {share}, call {call}: {rows.size} rows differ, the first is {rows[0]}"
         assert eng.device_status() == 0
         eng.close()
+
+
+@pytest.mark.parametrize("heads,ffn", [(4, 1024), (12, 3072)])
+def test_weights_given_to_the_layer_op_reach_whole_stack_calls(heads, ffn):
+    """A layer op that brings its own weights replaces the handle's.  The whole-stack calls run on weights with the
+    LayerNorms folded in: those have to follow, in passes recorded before as well, and also when only one layer of
+    the stack is replaced."""
+    layers, batch, seq, h = 3, 5, 24, heads * 64
+    rng = np.random.RandomState(3)
+    mask = torch.from_numpy(W.prefix_mask(rng.randint(1, seq + 1, size=batch).astype(np.int32), seq)).cuda()
+    x = torch.from_numpy(rng.randn(batch, seq, h).astype(np.float16)).cuda()
+    old, new = list(make_weights(layers, h, ffn, 1)), list(make_weights(layers, h, ffn, 2))
+
+    def engine(weights):
+        eng = et.EffectiveTransformer(layers, heads, 64, ffn, batch, seq, dtype=torch.float16)
+        for layer, w in enumerate(weights):
+            eng.set_layer_weights(layer, [t.cpu() for t in w])
+        return eng
+
+    def layer_op(eng, layer, w, packed, count, batch_idx, word_idx):
+        out = torch.empty_like(packed)
+        names = ["attr_kernel_Q", "attr_bias_Q", "attr_kernel_K", "attr_bias_K", "attr_kernel_V", "attr_bias_V",
+                 "attr_output_kernel", "attr_output_bias", "attr_output_layernorm_beta", "attr_output_layernorm_gamma",
+                 "inter_kernel", "inter_bias", "output_kernel", "output_bias", "output_layernorm_beta",
+                 "output_layernorm_gamma"]
+        p = _capi.EncoderParam()
+        for name, t in zip(names, w):
+            setattr(p, name, t.data_ptr())
+        p.from_tensor, p.to_tensor, p.transformer_out = packed.data_ptr(), packed.data_ptr(), out.data_ptr()
+        p.batch_idx, p.word_idx = batch_idx.data_ptr(), word_idx.data_ptr()
+        p.valid_word_num, p.stream = count.data_ptr(), torch.cuda.current_stream().cuda_stream
+        tp = _capi.TransformerParam(batch, seq, seq, heads, 64)
+        _capi.check(_capi.load().et_layer(eng._h, layer, C.byref(p), C.byref(tp)), eng._h)
+        return out
+
+    fresh = engine(new)
+    mixed = engine([old[0], new[1], old[2]])
+    want_new, want_mixed = fresh.forward(x, mask), mixed.forward(x, mask)
+    eng = engine(old)
+    out = torch.empty_like(x)
+    eng.capture(x, mask, out)
+    packed = eng.effective_transformer_input(x, mask)
+    layer_op(eng, 1, new[1], *packed)
+    assert torch.equal(eng.forward(x, mask), want_mixed)
+    eng.replay()
+    assert torch.equal(out, want_mixed)
+    for layer in (0, 2):
+        layer_op(eng, layer, new[layer], *packed)
+    assert torch.equal(eng.forward(x, mask), want_new)
+    eng.replay()
+    assert torch.equal(out, want_new)
+    for e in (fresh, mixed, eng):
+        e.close()
