@@ -125,7 +125,9 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
   };
   // Thread 0: Q block q0 (optional) and K/V block k0 of an item -> buffer at
   // `buf_addr`, completion on `bar`.  An empty item still arrives once.
+  uint32_t phases[3] = {0u, 0u, 0u};  // thread 0: started on each barrier, for a CTA that gives up
   auto issue = [&](const Item& it, uint32_t buf_addr, int q0, int k0, bool with_q, uint32_t bar) {
+    ++phases[(bar - bar0) >> 3];
     const int bq = (with_q && it.len > q0) ? (min(kBlock, it.len - q0) + kBoxRows - 1) / kBoxRows : 0;
     const int bk = it.len > k0 ? (min(kBlock, it.len - k0) + kBoxRows - 1) / kBoxRows : 0;
     mbar_arrive_expect_tx(bar, static_cast<uint32_t>((bq + 2 * bk) * kBoxBytes));
@@ -343,6 +345,9 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
     if (threadIdx.x == 0) fence_proxy_async_smem();
     cur = nxt;
   }
+  if (!ok && threadIdx.x == 0)  // copies in flight land before the shared memory goes away
+    for (int j = 0; j < 3; ++j)
+      if (phases[j] > 0) mbar_drain(bar0 + 8 * j, (phases[j] - 1) & 1u);
 }
 
 }  // namespace

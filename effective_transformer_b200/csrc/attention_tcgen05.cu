@@ -266,6 +266,15 @@ mask_bits_kernel(const __half* attr_mask, const int* batch_idx,
   }
 }
 
+// A CTA that gives up: its copies and MMAs in flight land before its shared memory and TMEM go away.  Arguments:
+// how many phases of each barrier have been started.
+__device__ __forceinline__ void drain_attention(uint32_t bar_qk, uint32_t qk, uint32_t bar_v, uint32_t v, uint32_t bar_mma,
+                                                uint32_t mma) {
+  if (qk > 0) mbar_drain(bar_qk, (qk - 1) & 1u);
+  if (v > 0) mbar_drain(bar_v, (v - 1) & 1u);
+  if (mma > 0) mbar_drain(bar_mma, (mma - 1) & 1u);
+}
+
 template <bool kMask>
 __global__ void __launch_bounds__(kThreads, kCtasPerSm)
 attention_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_k,
@@ -322,6 +331,7 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_q, const __gri
   const int total = num_tiles * heads;  // a CTA beyond it runs no item and frees its TMEM below
 
   uint32_t mma_phase = 0;
+  uint32_t qk_issued = 0, v_issued = 0, mma_issued = 0;  // thread 0: what a CTA that gives up has to see land
   bool ok = true;
   // Thread 0: Q and K rows of an item (barrier bar_qk) / its V rows (barrier bar_v).
   const uint32_t bar_qk = bar_load0, bar_v = bar_load0 + 8u;
@@ -329,6 +339,7 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_q, const __gri
   auto issue_qk = [&](int head_i, int first_row, int rows) {
     const int boxes = (clamp_rows(rows) + kBoxRows - 1) / kBoxRows;
     mbar_arrive_expect_tx(bar_qk, static_cast<uint32_t>(2 * boxes * kBoxBytes));
+    ++qk_issued;
     const int x = head_i * co.x_per_head, y = head_i * co.y_per_head + first_row;
     for (int j = 0; j < boxes; ++j) {
       tma_load_2d(base + j * kBoxBytes, &tmap_q, x, y + j * kBoxRows, bar_qk);
@@ -338,6 +349,7 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_q, const __gri
   auto issue_v = [&](int head_i, int first_row, int rows) {
     const int boxes = (clamp_rows(rows) + kBoxRows - 1) / kBoxRows;
     mbar_arrive_expect_tx(bar_v, static_cast<uint32_t>(boxes * kBoxBytes));
+    ++v_issued;
     const int x = head_i * co.x_per_head, y = head_i * co.y_per_head + first_row;
     for (int j = 0; j < boxes; ++j)
       tma_load_2d(base + 2 * kTileBytes + j * kBoxBytes, &tmap_v, x, y + j * kBoxRows, bar_v);
@@ -453,6 +465,7 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_q, const __gri
 #pragma unroll
       for (int k = 0; k < kD / 16; ++k) umma_f16_ss(tmem_base, qd + 2u * k, kd + 2u * k, idesc, k != 0 ? 1u : 0u);
       umma_commit(bar_mma);
+      ++mma_issued;
     }
     ItemMeta nxt;
     meta_tile(item + static_cast<int>(gridDim.x), nxt);
@@ -560,6 +573,7 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_q, const __gri
         umma_f16_ts(tmem_base + kOCol, tmem_base + kPCol + ks * 8, vd, idesc, ks != 0 ? 1u : 0u);
       }
       umma_commit(bar_mma);
+      ++mma_issued;
     }
     meta_row(nxt);
     ok = wait_all(bar_mma, mma_phase, kSiteContext);
@@ -599,6 +613,7 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_q, const __gri
     meta_finish(nxt);
     cur = nxt;
   }
+  if (!ok && threadIdx.x == 0) drain_attention(bar_qk, qk_issued, bar_v, v_issued, bar_mma, mma_issued);
 
   tc_fence_before();
   __syncthreads();
@@ -683,7 +698,7 @@ attention_tcgen05_long_kernel(const __grid_constant__ CUtensorMap tmap_q, const 
       }
       return __syncthreads_and(got) != 0;
     };
-    int qk_issued = 0, v_issued = 0, qk_seen = 0, v_seen = 0;  // copies requested / waited for
+    uint32_t qk_issued = 0, v_issued = 0, mma_issued = 0;  // thread 0: what a CTA that gives up has to see land
     if (threadIdx.x == 0) {
       const int bq = boxes_of(q0), bk = boxes_of(0);
       mbar_arrive_expect_tx(bar_qk, static_cast<uint32_t>((bq + bk) * kBoxBytes));
@@ -691,8 +706,8 @@ attention_tcgen05_long_kernel(const __grid_constant__ CUtensorMap tmap_q, const 
       load_rows(sk, &tmap_k, 0, bk, bar_qk);
       mbar_arrive_expect_tx(bar_v, static_cast<uint32_t>(bk * kBoxBytes));
       load_rows(sv, &tmap_v, 0, bk, bar_v);
+      qk_issued = v_issued = 1;
     }
-    qk_issued = v_issued = 1;
 
     const bool warp_has_rows = warp * 32 < nq;
     float o[kD];
@@ -707,7 +722,6 @@ attention_tcgen05_long_kernel(const __grid_constant__ CUtensorMap tmap_q, const 
       const bool has_next = j + 1 < k_tiles;
       ok = wait_all(bar_qk, static_cast<uint32_t>(j & 1), kSiteLoad);
       if (!ok) break;
-      ++qk_seen;
       // ---- S = Q K^T ----
       if (threadIdx.x == 0) {
         tc_fence_after();
@@ -716,6 +730,7 @@ attention_tcgen05_long_kernel(const __grid_constant__ CUtensorMap tmap_q, const 
 #pragma unroll
         for (int k = 0; k < kD / 16; ++k) umma_f16_ss(tmem_base, qd + 2u * k, kd + 2u * k, idesc, k != 0 ? 1u : 0u);
         umma_commit(bar_mma);
+        ++mma_issued;
       }
       ok = wait_all(bar_mma, mma_phase, kSiteScores);
       mma_phase ^= 1u;
@@ -726,8 +741,8 @@ attention_tcgen05_long_kernel(const __grid_constant__ CUtensorMap tmap_q, const 
           const int bk = boxes_of((j + 1) * kTileRows);
           mbar_arrive_expect_tx(bar_qk, static_cast<uint32_t>(bk * kBoxBytes));
           load_rows(sk, &tmap_k, (j + 1) * kTileRows, bk, bar_qk);
+          ++qk_issued;
         }
-        ++qk_issued;
       }
       float corr = 1.f;
       if (warp_has_rows) {
@@ -793,7 +808,6 @@ attention_tcgen05_long_kernel(const __grid_constant__ CUtensorMap tmap_q, const 
       tc_fence_before();
       ok = __syncthreads_and(got_v) != 0;
       if (!ok) break;
-      ++v_seen;
       // ---- O_j = P V ----
       if (threadIdx.x == 0) {
         tc_fence_after();
@@ -803,6 +817,7 @@ attention_tcgen05_long_kernel(const __grid_constant__ CUtensorMap tmap_q, const 
           umma_f16_ts(tmem_base + kOCol, tmem_base + kPCol + ks * 8, vd, idesc, ks != 0 ? 1u : 0u);
         }
         umma_commit(bar_mma);
+        ++mma_issued;
       }
       ok = wait_all(bar_mma, mma_phase, kSiteContext);
       mma_phase ^= 1u;
@@ -814,8 +829,8 @@ attention_tcgen05_long_kernel(const __grid_constant__ CUtensorMap tmap_q, const 
           const int bk = boxes_of((j + 1) * kTileRows);
           mbar_arrive_expect_tx(bar_v, static_cast<uint32_t>(bk * kBoxBytes));
           load_rows(sv, &tmap_v, (j + 1) * kTileRows, bk, bar_v);
+          ++v_issued;
         }
-        ++v_issued;
       }
       if (warp_has_rows) {
 #pragma unroll
@@ -842,10 +857,7 @@ attention_tcgen05_long_kernel(const __grid_constant__ CUtensorMap tmap_q, const 
                      : "memory");
       }
     }
-    if (threadIdx.x == 0 && !ok) {  // copies in flight must land before the shared memory goes away
-      if (qk_issued > qk_seen) mbar_wait(bar_qk, static_cast<uint32_t>((qk_issued - 1) & 1), abort_flag);
-      if (v_issued > v_seen) mbar_wait(bar_v, static_cast<uint32_t>((v_issued - 1) & 1), abort_flag);
-    }
+    if (!ok && threadIdx.x == 0) drain_attention(bar_qk, qk_issued, bar_v, v_issued, bar_mma, mma_issued);
   }
 
   tc_fence_before();

@@ -219,7 +219,7 @@ gemm_split_kernel(const __grid_constant__ Maps maps, void* __restrict__ c_ptr, f
             fail(kSiteDrain);
       // copies in flight must land before the CTA's shared memory goes away
       for (int i = max(0, issued - S); i < issued; ++i)
-        if (!mbar_wait(full_bar(i % S), static_cast<uint32_t>((i / S) & 1), abort_flag) && *abort_flag == 0)
+        if (!mbar_drain(full_bar(i % S), static_cast<uint32_t>((i / S) & 1)) && *abort_flag == 0)
           fail(kSiteDrain);
     } else {
       pdl_wait();
@@ -266,7 +266,7 @@ gemm_split_kernel(const __grid_constant__ Maps maps, void* __restrict__ c_ptr, f
       }
       if (ok) umma_commit(acc_bar);
       umma_commit(drain_bar);
-      if (!mbar_wait(drain_bar, 0u, abort_flag) && *abort_flag == 0) fail(kSiteMmaDrain);
+      if (!mbar_drain(drain_bar, 0u) && *abort_flag == 0) fail(kSiteMmaDrain);
     }
     __syncwarp();
     if (splits > 1) {

@@ -523,8 +523,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a,
       const long long pending = issued < S ? issued : S;
       for (long long i = 0; i < pending; ++i) {
         const long long f = issued - 1 - i;
-        if (!mbar_wait(full_bar(static_cast<int>(f % S)), static_cast<uint32_t>((f / S) & 1),
-                       abort_flag) && *abort_flag == 0)
+        if (!mbar_drain(full_bar(static_cast<int>(f % S)), static_cast<uint32_t>((f / S) & 1)) && *abort_flag == 0)
           fail(kSiteProducerDrain);
       }
     }
@@ -569,7 +568,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a,
       }
       // All MMAs must have retired before TMEM is freed.
       umma_commit(drain_bar);
-      if (!mbar_wait(drain_bar, 0u, abort_flag) && *abort_flag == 0) fail(kSiteMmaDrain);
+      if (!mbar_drain(drain_bar, 0u) && *abort_flag == 0) fail(kSiteMmaDrain);
     }
   } else {
     // ------------------------- epilogue -------------------------
@@ -803,8 +802,7 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap tmap_a,
         const long long pending = issued < S ? issued : S;
         for (long long i = 0; i < pending; ++i) {
           const long long f = issued - 1 - i;
-          if (!mbar_wait(full_bar(static_cast<int>(f % S)), static_cast<uint32_t>((f / S) & 1),
-                         abort_flag) && *abort_flag == 0)
+          if (!mbar_drain(full_bar(static_cast<int>(f % S)), static_cast<uint32_t>((f / S) & 1)) && *abort_flag == 0)
             fail(kSiteProducerDrain);
         }
       }
@@ -853,7 +851,7 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap tmap_a,
         }
       }
       umma_commit_pair(drain_bar);
-      if (!mbar_wait(drain_bar, 0u, abort_flag) && *abort_flag == 0) fail(kSiteMmaDrain);
+      if (!mbar_drain(drain_bar, 0u) && *abort_flag == 0) fail(kSiteMmaDrain);
     }
   } else if (warp < 2 + kEpilogueWarps) {
     // ------------------------- epilogue (both CTAs) -------------------------

@@ -337,7 +337,7 @@ gemm_tf32x3_kernel(const __grid_constant__ CUtensorMap tmap_a_hi, const __grid_c
       const long long pending = issued < S ? issued : S;
       for (long long i = 0; i < pending; ++i) {
         const long long f = issued - 1 - i;
-        if (!mbar_wait(full_bar(static_cast<int>(f % S)), static_cast<uint32_t>((f / S) & 1), abort_flag) &&
+        if (!mbar_drain(full_bar(static_cast<int>(f % S)), static_cast<uint32_t>((f / S) & 1)) &&
             *abort_flag == 0)
           fail(kSiteProducerDrain);
       }
@@ -391,7 +391,7 @@ gemm_tf32x3_kernel(const __grid_constant__ CUtensorMap tmap_a_hi, const __grid_c
         }
       }
       umma_commit(drain_bar);  // all MMAs must have retired before TMEM is freed
-      if (!mbar_wait(drain_bar, 0u, abort_flag) && *abort_flag == 0) fail(kSiteMmaDrain);
+      if (!mbar_drain(drain_bar, 0u) && *abort_flag == 0) fail(kSiteMmaDrain);
     }
   } else {
     // ------------------------- epilogue -------------------------
@@ -621,7 +621,7 @@ gemm_tf32x3_pair_kernel(const __grid_constant__ CUtensorMap tmap_a_hi, const __g
         const long long pending = issued < S ? issued : S;
         for (long long i = 0; i < pending; ++i) {
           const long long f = issued - 1 - i;
-          if (!mbar_wait(full_bar(static_cast<int>(f % S)), static_cast<uint32_t>((f / S) & 1), abort_flag) &&
+          if (!mbar_drain(full_bar(static_cast<int>(f % S)), static_cast<uint32_t>((f / S) & 1)) &&
               *abort_flag == 0)
             fail(kSiteProducerDrain);
         }
@@ -681,7 +681,7 @@ gemm_tf32x3_pair_kernel(const __grid_constant__ CUtensorMap tmap_a_hi, const __g
         }
       }
       umma_commit_pair(drain_bar);
-      if (!mbar_wait(drain_bar, 0u, abort_flag) && *abort_flag == 0) fail(kSiteMmaDrain);
+      if (!mbar_drain(drain_bar, 0u) && *abort_flag == 0) fail(kSiteMmaDrain);
     }
   } else {
     // ------------------------- epilogue (both CTAs) -------------------------

@@ -82,6 +82,18 @@ __device__ __forceinline__ bool mbar_wait_ns(uint32_t bar, uint32_t parity, vola
 __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatile int* abort_flag) {
   return mbar_wait_ns(bar, parity, abort_flag, kWaitTimeoutNs);
 }
+// Wait for what this CTA has in flight itself (copies into its shared memory, MMAs that read it and write its
+// TMEM) before it gives that memory back.  It lands in microseconds whatever the other roles do, so the abort
+// flag, behind which mbar_wait returns at once, does not end this wait; only a CTA pair whose peer gave up can
+// leave a phase incomplete, hence the limit.
+constexpr unsigned long long kDrainTimeoutNs = 100000000ull;  // 100 ms
+__device__ __forceinline__ bool mbar_drain(uint32_t bar, uint32_t parity) {
+  const unsigned long long t0 = globaltimer_ns();
+  for (uint32_t spin = 1;; ++spin) {
+    if (mbar_try_wait(bar, parity)) return true;
+    if ((spin & 127u) == 0u && globaltimer_ns() - t0 > kDrainTimeoutNs) return false;
+  }
+}
 
 // ---- TMA --------------------------------------------------------------------
 __device__ __forceinline__ void prefetch_tensormap(const CUtensorMap* map) {

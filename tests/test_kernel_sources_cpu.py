@@ -69,3 +69,17 @@ def test_ring_commits_are_waited_for_before_the_barriers_go_away():
                 seen += 1
                 assert body.count("mbar_wait(empty_bar(") == 2, f"{name}: {kernel}"
     assert seen == 5
+
+
+def test_what_is_in_flight_lands_even_when_a_role_has_given_up():
+    """mbar_wait returns at once behind the abort flag, so it cannot be the wait that keeps shared memory and TMEM
+    until copies and MMAs in flight have landed."""
+    for name in FILES:
+        text = read(name)
+        for site in re.findall(r"if \(!(mbar_\w+)\((full_bar|drain_bar)[^;]*?fail\(kSite\w*Drain\)", text):
+            assert site[0] == "mbar_drain", f"{name}: {site}"
+    attention = dict((k, b) for k, _, b in kernels(read("attention_tcgen05.cu")))
+    for kernel in ("attention_tcgen05_kernel", "attention_tcgen05_long_kernel"):
+        body = attention[kernel]
+        assert "drain_attention(bar_qk, qk_issued, bar_v, v_issued, bar_mma, mma_issued)" in body
+        assert body.count("umma_commit(bar_mma);") == body.count("++mma_issued;") == 2
