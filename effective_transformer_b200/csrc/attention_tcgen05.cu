@@ -105,13 +105,15 @@ __host__ __device__ inline size_t plan_ints(int batch, int max_tokens) {
 // from cu_seqlens.  The boundaries are kept in shared memory: the binary search below is a chain of
 // dependent reads.
 // The op-by-op pass of the 100 x 32 batch, 12 layers: 1057 -> 1030 us with one kernel in place of two.
-constexpr int kSharedSeqs = 8128;
+constexpr int kSharedSeqs = 8192;
+// boundaries and next(), below
+constexpr int plan_smem_bytes(int batch) { return batch <= kSharedSeqs ? (batch + 1) * 4 + batch * 2 : 0; }
 __global__ void attention_plan_kernel(const int* cu_seqlens, const int* batch_idx,
                                       const int* t_ptr, int* __restrict__ cu_out, int batch,
                                       int max_tokens, int* __restrict__ plan) {
   pdl_wait();
   pdl_trigger();
-  __shared__ int s_cu[kSharedSeqs + 1];
+  extern __shared__ int s_cu[];  // [batch + 1], then uint16_t [batch]
   const bool shared_cu = batch <= kSharedSeqs;
   if (shared_cu) {
     if (batch_idx != nullptr) {
@@ -140,7 +142,7 @@ __global__ void attention_plan_kernel(const int* cu_seqlens, const int* batch_id
   // behind the tile's first token.  next() is found for every b in parallel (a
   // binary search over the sorted boundaries); only the walk along the chain,
   // one step per tile, is sequential.
-  __shared__ uint16_t s_next[kSharedSeqs];
+  uint16_t* s_next = reinterpret_cast<uint16_t*>(s_cu + batch + 1);
   const bool scratch_ok = shared_cu || batch <= max_tokens;  // larger batches: global scratch (slower walk)
   auto cu = [&](int b) { return min(bounds[b], max_tokens); };
   if (scratch_ok) {
@@ -889,16 +891,26 @@ bool qkv_coords(long long token_stride, long long head_stride, int heads, int ma
 
 }  // namespace
 
+namespace {
+cudaError_t launch_plan(const int* cu_seqlens, const int* batch_idx, const int* t_ptr, int* cu_out, int batch,
+                        int max_tokens, int* plan, cudaStream_t stream) {
+  if (batch <= 0) return cudaSuccess;
+  static PerDeviceOnce once;  // function attributes are per device
+  const cudaError_t once_err = once.run([] {
+    return cudaFuncSetAttribute(attention_plan_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                plan_smem_bytes(kSharedSeqs));
+  });
+  if (once_err != cudaSuccess) return once_err;
+  return launch_pdl(attention_plan_kernel, dim3(1), dim3(1024), plan_smem_bytes(batch), stream, cu_seqlens, batch_idx,
+                    t_ptr, cu_out, batch, max_tokens, plan);
+}
+}  // namespace
+
 size_t attention_plan_ints(int batch, int max_tokens) { return plan_ints(batch, max_tokens); }
 
 cudaError_t launch_attention_plan(const int* cu_seqlens, int batch, int max_tokens, int* plan,
                                   cudaStream_t stream) {
-  if (batch <= 0) return cudaSuccess;
-  const cudaError_t le = launch_pdl(attention_plan_kernel, dim3(1), dim3(1024), 0, stream, cu_seqlens,
-                                    static_cast<const int*>(nullptr), static_cast<const int*>(nullptr),
-                                    static_cast<int*>(nullptr), batch, max_tokens, plan);
-  if (le != cudaSuccess) return le;
-  return cudaGetLastError();
+  return launch_plan(cu_seqlens, nullptr, nullptr, nullptr, batch, max_tokens, plan, stream);
 }
 
 // Up to 16 384 rows the single CTA reads the sequence numbers in 16 coalesced rounds.
@@ -908,9 +920,7 @@ bool attention_plan_from_rows_supported(int batch, int max_tokens) {
 
 cudaError_t launch_attention_plan_from_rows(const int* batch_idx, const int* t_ptr, int batch, int max_tokens,
                                             int* cu_seqlens, int* plan, cudaStream_t stream) {
-  if (batch <= 0) return cudaSuccess;
-  return launch_pdl(attention_plan_kernel, dim3(1), dim3(1024), 0, stream, static_cast<const int*>(nullptr), batch_idx,
-                    t_ptr, cu_seqlens, batch, max_tokens, plan);
+  return launch_plan(nullptr, batch_idx, t_ptr, cu_seqlens, batch, max_tokens, plan, stream);
 }
 
 size_t attention_mask_bits_words(size_t max_tokens) { return max_tokens * kMaskBitsStride; }

@@ -117,3 +117,28 @@ def test_weights_given_to_the_layer_op_reach_whole_stack_calls(heads, ffn):
     assert torch.equal(out, want_new)
     for e in (fresh, mixed, eng):
         e.close()
+
+
+@pytest.mark.parametrize("batch", [8190, 8191, 8192, 8193])
+def test_attention_plan_of_thousands_of_short_sequences(batch):
+    """Up to 8192 sequences the boundaries and the packing chain are kept in shared memory (from 8191 on more of it
+    than a kernel has without asking); beyond, in global memory."""
+    seq, heads = 2, 2
+    lens = np.random.RandomState(batch).randint(0, seq + 1, size=batch).astype(np.int32)
+    lens[0], lens[-1] = 0, 1
+    mask = torch.from_numpy(W.prefix_mask(lens, seq)).cuda()
+    gen = torch.Generator(device="cuda").manual_seed(batch)
+    x = torch.randn(batch, seq, heads * 64, device="cuda", dtype=torch.float16, generator=gen)
+    eng = make_engine(1, batch, seq, heads, 256)
+    exact = make_engine(1, batch, seq, heads, 256, dtype=torch.float32)
+    got = eng.forward(x, mask)
+    ops = et.get_sequence_output(et.BertConfig(heads * 64, 1, heads, 256), batch, seq, None, mask, x, None, engine=eng)
+    want = exact.forward(x.float(), mask)
+    rows = mask.bool()
+    for y in (got, ops):
+        err = (y.float() - want)[rows].norm(dim=1) / want[rows].norm(dim=1)
+        assert float(err.max()) < 4e-3  # one layer of fp16 roundings (2^-11 each) on rows of LayerNorm outputs
+        assert not y[~rows].any()
+    assert eng.device_status() == 0
+    eng.close()
+    exact.close()
