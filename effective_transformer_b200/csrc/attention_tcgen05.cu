@@ -234,7 +234,7 @@ struct MaskArgs {
 // positions it may attend to, as a float.  A warp per token, lanes over the row's keys, so that a mask row is
 // read in whole lines; in the attention kernel a thread reads its row alone, twice, key by key, and again for
 // every head of every layer.
-constexpr int kMaskBitsStride = 8;
+constexpr int kMaskBitsStride = kMaskBitsBytes / 4;
 __global__ void __launch_bounds__(256)
 mask_bits_kernel(const __half* attr_mask, const int* batch_idx,
                  const int* word_idx, const int* cu_seqlens, const int* t_ptr,
@@ -922,8 +922,6 @@ cudaError_t launch_attention_plan_from_rows(const int* batch_idx, const int* t_p
                                             int* cu_seqlens, int* plan, cudaStream_t stream) {
   return launch_plan(nullptr, batch_idx, t_ptr, cu_seqlens, batch, max_tokens, plan, stream);
 }
-
-size_t attention_mask_bits_words(size_t max_tokens) { return max_tokens * kMaskBitsStride; }
 
 cudaError_t launch_attention_mask_bits(const __half* attr_mask, const int* batch_idx, const int* word_idx,
                                        const int* cu_seqlens, const int* t_ptr, int max_tokens, int seq,

@@ -410,7 +410,7 @@ cudaError_t launch_attention_tcgen05(const __half* q, const __half* k, const __h
                                      const int* batch_idx = nullptr, const int* word_idx = nullptr, int seq = 0,
                                      const uint32_t* mask_bits = nullptr);
 // The general mask as bits per token, once per batch, for the launches of its layers (mask_bits above).
-size_t attention_mask_bits_words(size_t max_tokens);
+constexpr int kMaskBitsBytes = 32;  // per token
 cudaError_t launch_attention_mask_bits(const __half* attr_mask, const int* batch_idx, const int* word_idx,
                                        const int* cu_seqlens, const int* t_ptr, int max_tokens, int seq,
                                        uint32_t* bits, cudaStream_t stream);

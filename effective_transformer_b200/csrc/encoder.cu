@@ -103,7 +103,9 @@ struct Workspace {
   int* lens_scratch = nullptr;
   int* attn_plan = nullptr;   // tile plan of the tcgen05 attention (made once per batch)
   int* pos_row = nullptr;     // [B*S] position -> packed row (general-mask attention)
-  uint32_t* mask_bits = nullptr;  // a general mask as bits per token (attention on packed tiles)
+  // A general mask as bits per token (attention on packed tiles) lies in stage_out: only the host-buffer calls use
+  // that, they take no general mask, and two calls of a handle share x, qkv, ... and so never overlap anyway.
+  uint32_t* mask_bits() const { return static_cast<uint32_t*>(stage_out); }
   float* a_hi = nullptr;      // fp32 handles: [cap, H] tf32 halves of a projection's input
   float* a_lo = nullptr;
   float* ffn_lo = nullptr;    // fp32 handles: [cap, F] remainder of the GELU output (its tf32 half is in ffn)
@@ -151,7 +153,6 @@ std::vector<WsItem> workspace_items(const et_config_t& c, size_t batch, size_t s
       {I(&ws.lens_scratch), batch * 4},
       {I(&ws.attn_plan), attention_plan_ints(static_cast<int>(batch), static_cast<int>(cap)) * 4},
       {I(&ws.pos_row), cap * 4},
-      {reinterpret_cast<void**>(&ws.mask_bits), f32 ? 0 : attention_mask_bits_words(cap) * 4},
       {F(&ws.a_hi), f32 ? cap * H * 4 : 0}, {F(&ws.a_lo), f32 ? cap * H * 4 : 0},
       {F(&ws.ffn_lo), f32 ? cap * f * 4 : 0},
       {I(&ws.ln_counters), ln_counter_ints(bs) * 4},
@@ -216,7 +217,7 @@ struct et_handle_s {
   const void* cur_attr_mask = nullptr;
   const int* cur_word_idx = nullptr;
   const int* cur_batch_idx = nullptr;
-  bool mask_bits_ready = false;  // ws.mask_bits holds that mask (inside a whole-stack call)
+  bool mask_bits_ready = false;  // ws.mask_bits() holds that mask (inside a whole-stack call)
   // Rows by which the projections' kernels are chosen, 0 = the pass's own capacity.  A host-buffer call sets the
   // whole batch's for the passes over its chunks: their shares follow measured times, the result must not.
   int route_rows = 0;
@@ -552,7 +553,7 @@ int run_layer(et_handle_t h, const LayerWeights& lw, const T* x_in, T* x_out, co
                                        reinterpret_cast<__half*>(ctx), ws.attn_plan, batch, max_m, heads, d,
                                        ws.status, s, turn(), &h->maps,
                                        static_cast<const __half*>(h->cur_attr_mask), h->cur_batch_idx,
-                                       h->cur_word_idx, seq, h->mask_bits_ready ? ws.mask_bits : nullptr));
+                                       h->cur_word_idx, seq, h->mask_bits_ready ? ws.mask_bits() : nullptr));
   else if (masked)
     ET_LAUNCH(h, ET_PROF_ATTENTION, 1, s,
               launch_attention_masked_simt<T>(qkv, qkv + hid, qkv + 2 * hid, 3LL * hid, d, ctx,
@@ -778,9 +779,11 @@ int stack_impl(et_handle_t h, int batch, int seq, cudaStream_t s) {
     ET_LAUNCH(h, ET_PROF_PADDING_OFFSETS, 1, s,
               launch_attention_plan(ws.cu_seqlens, batch, max_m, ws.attn_plan, s));
   if (tiles && h->cur_attr_mask != nullptr) {
+    // (a row of stage_out is hidden * 2 bytes, 256 at least; a token's bits are 32)
+    static_assert(kMaskBitsBytes <= 256, "the bits of a token must fit a row of stage_out");
     ET_LAUNCH(h, ET_PROF_PADDING_OFFSETS, 1, s,
               launch_attention_mask_bits(static_cast<const __half*>(h->cur_attr_mask), h->cur_batch_idx,
-                                         h->cur_word_idx, ws.cu_seqlens, ws.valid_word_num, max_m, seq, ws.mask_bits,
+                                         h->cur_word_idx, ws.cu_seqlens, ws.valid_word_num, max_m, seq, ws.mask_bits(),
                                          s));
     h->mask_bits_ready = true;  // (MaskScope, which set the mask, clears it)
   } else if (!tiles && h->cur_attr_mask != nullptr)

@@ -142,3 +142,30 @@ def test_attention_plan_of_thousands_of_short_sequences(batch):
     assert eng.device_status() == 0
     eng.close()
     exact.close()
+
+
+def test_no_workspace_is_held_for_general_masks():
+    """The bits of a general mask lie in a buffer that only the host-buffer calls use otherwise: a handle pays
+    nothing for them, and the two kinds of calls on one handle do not disturb each other."""
+    batch, seq, heads, ffn = 24, 40, 4, 1024
+    h = heads * 64
+    eng = make_engine(2, batch, seq, heads, ffn)
+    per_position = (eng.workspace_bytes(batch, 128 * seq) - eng.workspace_bytes(batch, 64 * seq)) / (batch * 64 * seq)
+    activations = 2 * (8 * h + ffn)             # x, qkv, ctx, att, two staging buffers; ffn
+    indices = 4 * 10                            # masks, ids, types, four index arrays, two plan labels, position rows
+    statistics = 2 * 8 * (h // 64) + 0.125      # deferred LayerNorm; row counters
+    assert per_position <= activations + indices + statistics + 1
+    rng = np.random.RandomState(4)
+    lens = rng.randint(1, seq + 1, size=batch).astype(np.int32)
+    mask_np = W.prefix_mask(lens, seq)
+    x_np = rng.randn(batch, seq, h).astype(np.float16)
+    x, mask = torch.from_numpy(x_np).cuda(), torch.from_numpy(mask_np).cuda()
+    causal = torch.tril(torch.ones(batch, seq, seq, device="cuda", dtype=torch.float16))
+    masked, plain = eng.forward_general_mask(x, mask, causal).clone(), eng.forward(x, mask).cpu().numpy()
+    for _ in range(3):
+        got, _ = eng.forward_host(x_np, mask_np)
+        assert np.array_equal(got, plain)
+        again = eng.forward_general_mask(x, mask, causal)
+        torch.cuda.synchronize()  # (a host call runs on the handle's own stream)
+        assert torch.equal(again, masked)
+    eng.close()
