@@ -90,6 +90,7 @@ SIGNATURES = {
     "et_selftest_wait_timeout": (i32, [vp, vp]),
     "et_workspace_allocated_bytes": (i32, [vp, C.POINTER(C.c_size_t)]),
     "et_gemm_fused": (i32, [vp, vp, vp, vp, vp, vp, C.c_float, vp, vp, vp, i32, i32, i32, i32, vp, vp]),
+    "et_gemm_route": (i32, [i32, i32, i32, i32, i32, ip, ip]),
     "et_fold_layernorm": (i32, [vp, vp, vp, vp, vp, vp, vp, i32, i32, vp]),
     "et_gemm_deferred_norm": (i32, [vp, vp, vp, vp, vp, vp, vp, C.c_float, vp, vp, vp, vp, i32, i32, i32, i32, vp, vp]),
     "et_padding_offsets": (i32, [vp, i32, i32, vp, vp, vp, vp, vp, vp, vp, vp, vp]),

@@ -463,7 +463,8 @@ struct SplitPlan {
   int bn = 64;
   int splits = 0;
 };
-SplitPlan gemm_split_plan(int max_m, int n, int k, bool tf32, bool feeds_attention = false);
+// The plan of a projection of `rows` rows (a capacity) with this epilogue.
+SplitPlan gemm_route(bool tf32, int rows, int n, int k, int epilogue);
 cudaError_t launch_gemm_split(const SplitGemm& g, int epilogue, const SplitPlan& plan, TensorMapCache* maps,
                               cudaStream_t stream);
 // Whether the fused LayerNorm epilogues can serve a projection of n output columns.

@@ -2141,6 +2141,16 @@ int et_fold_layernorm(const void* w_packed, const void* bias, const void* gamma,
                                          static_cast<cudaStream_t>(stream)));
 }
 
+int et_gemm_route(int dtype, int rows, int n, int k, int epilogue, int* tile_n, int* splits) {
+  if ((dtype != ET_FP16 && dtype != ET_FP32) || rows <= 0 || n <= 0 || k <= 0 || n % 128 != 0 || k % 8 != 0 ||
+      epilogue < kEpiNone || epilogue > kEpiNormResidual || !tile_n || !splits)
+    return ET_INVALID_ARGUMENT;
+  const SplitPlan p = gemm_route(dtype == ET_FP32, rows, n, k, epilogue);
+  *splits = p.splits;
+  *tile_n = p.splits != 0 ? p.bn : n % 256 == 0 ? 256 : 128;
+  return ET_OK;
+}
+
 int et_gemm_deferred_norm(const void* a, const void* w_packed, const void* bias, const void* csum,
                           const void* residual, const void* gamma, const void* beta, float eps,
                           const float* stats_in, float* stats_out, void* c, const int* m_ptr, int max_m, int n,

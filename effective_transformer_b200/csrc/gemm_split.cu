@@ -555,7 +555,7 @@ bool encode_split(CUtensorMap* map, bool tf32, const void* base, int rows, int k
 // or 48 KB per 32-wide step, a 128-wide tile's longer reduction counted as another 128 KB.  From six row tiles on a
 // third more CTAs than SMs is taken where K is long: a batch has padding, and the tiles it leaves empty cost next
 // to nothing (N = 768, K = 3072, capacity 1024: 1591 against 1727; full, the launch alone 44 us against 54).
-SplitPlan gemm_split_plan(int max_m, int n, int k, bool tf32, bool feeds_attention) {
+static SplitPlan gemm_split_plan(int max_m, int n, int k, bool tf32, bool feeds_attention) {
   SplitPlan best;
   if (max_m <= 0) return best;
   const int num_kb = (k + (tf32 ? 31 : 63)) / (tf32 ? 32 : 64);
@@ -603,6 +603,13 @@ SplitPlan gemm_split_plan(int max_m, int n, int k, bool tf32, bool feeds_attenti
     if (best.splits != 0) break;
   }
   return best;
+}
+
+SplitPlan gemm_route(bool tf32, int rows, int n, int k, int epilogue) {
+  // the LayerNorm inside the GEMM kernel is the persistent kernel's
+  if (epilogue == kEpiResidualLayerNorm || epilogue == kEpiLayerNorm) return SplitPlan();
+  // the QKV projection is the one without activation or residual behind its bias
+  return gemm_split_plan(rows, n, k, tf32, !tf32 && (epilogue == kEpiBias || epilogue == kEpiNormIn));
 }
 
 cudaError_t launch_gemm_split(const SplitGemm& g, int epilogue, const SplitPlan& plan, TensorMapCache* maps, cudaStream_t stream) {

@@ -1377,11 +1377,7 @@ cudaError_t launch_gemm_tcgen05(const __half* a, const __half* w_packed, const _
     }
     lnp = *ln;
   }
-  // the QKV projection is the one without activation or residual behind its bias
-  const bool feeds_attention = epilogue == kEpiBias || epilogue == kEpiNormIn;
-  if (route_rows <= 0) route_rows = max_m;
-  if (const SplitPlan plan = has_ln(epilogue) ? SplitPlan() : gemm_split_plan(route_rows, n, k, false, feeds_attention);
-      plan.splits != 0) {
+  if (const SplitPlan plan = gemm_route(false, route_rows > 0 ? route_rows : max_m, n, k, epilogue); plan.splits != 0) {
     SplitGemm g;
     g.a = a, g.w = w_packed, g.bias = bias, g.residual = residual, g.c = c;
     g.m_ptr = m_ptr, g.max_m = max_m, g.n = n, g.k = k;

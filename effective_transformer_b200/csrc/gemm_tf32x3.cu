@@ -834,7 +834,7 @@ cudaError_t launch_gemm_tf32x3(const float* a_hi, const float* a_lo, const float
   if (bias != nullptr && (reinterpret_cast<uintptr_t>(bias) & 15u)) return cudaErrorMisalignedAddress;
   if (c_lo != nullptr && (reinterpret_cast<uintptr_t>(c_lo) & 15u)) return cudaErrorMisalignedAddress;
   if (epilogue != kEpiNone && bias == nullptr) return cudaErrorInvalidValue;
-  if (const SplitPlan plan = gemm_split_plan(route_rows > 0 ? route_rows : max_m, n, k, true); plan.splits != 0) {
+  if (const SplitPlan plan = gemm_route(true, route_rows > 0 ? route_rows : max_m, n, k, epilogue); plan.splits != 0) {
     SplitGemm g;
     g.a = a_hi, g.a_lo = a_lo, g.w = w_hi, g.w_lo = w_lo, g.bias = bias, g.c = c, g.c_lo = c_lo;
     g.m_ptr = m_ptr, g.max_m = max_m, g.n = n, g.k = k;

@@ -557,6 +557,12 @@ int et_gemm_deferred_norm(const void* a, const void* w_packed, const void* bias,
                           const float* stats_in, float* stats_out, void* c, const int* m_ptr, int max_m, int n,
                           int k, int epilogue, int* status_word, void* stream);
 
+/* Which kernel a projection of `rows` rows (the capacity: the valid rows are only
+ * known on the device) with this epilogue runs: splits = 0, the persistent kernels;
+ * otherwise tiles of 128 x *tile_n whose K range `splits` CTAs share.  Host only, on the current
+ * device's SM count (148 without a device).  No reference counterpart. */
+int et_gemm_route(int dtype, int rows, int n, int k, int epilogue, int* tile_n, int* splits);
+
 /* The same call sites for the FP32 OperationType on the tensor cores, keeping
  * fp32 accuracy: every operand is split into two tf32 numbers, x = hi + lo with
  * hi = round_to_tf32(x) (et_split_tf32; hi or lo may be x itself), and the
