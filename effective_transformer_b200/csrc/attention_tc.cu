@@ -72,15 +72,9 @@ struct Item {
   int lo, len, head;
 };
 
-// How (token, head) maps to TMA coordinates: x = head * x_per_head,
-// y = head * y_per_head + token.
-struct Coords {
-  int x_per_head, y_per_head;
-};
-
 __global__ void __launch_bounds__(kThreads, kCtasPerSm)
 attention_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_k,
-                    const __grid_constant__ CUtensorMap tmap_v, Coords co, __half* __restrict__ ctx,
+                    const __grid_constant__ CUtensorMap tmap_v, QkvCoords co, __half* __restrict__ ctx,
                     const int* __restrict__ cu_seqlens, int batch, int heads, int max_seq,
                     float scale_log2e, int* status_word) {
   extern __shared__ __align__(1024) uint8_t smem_raw[];
@@ -366,25 +360,9 @@ cudaError_t launch_attention_tc(const __half* q, const __half* k, const __half* 
   if (attention_long_supported(ctx, max_seq))
     return launch_attention_tcgen05_long(q, k, v, token_stride, head_stride, ctx, cu_seqlens, batch, max_seq, max_tokens,
                                          heads, d, status_word, stream, maps);
-  // Two layouts: heads side by side inside a token row (x moves with the head),
-  // or one [max_tokens, 64] block per head (y moves with the head).
-  Coords co;
-  uint64_t cols, rows;
-  if (static_cast<long long>(heads - 1) * head_stride + kD <= token_stride) {
-    co = {static_cast<int>(head_stride), 0};
-    cols = static_cast<uint64_t>(heads - 1) * head_stride + kD;
-    rows = static_cast<uint64_t>(max_tokens);
-  } else if (token_stride == kD && head_stride % token_stride == 0 && head_stride / token_stride >= max_tokens) {
-    co = {0, static_cast<int>(head_stride / token_stride)};
-    cols = kD;
-    rows = static_cast<uint64_t>(heads - 1) * (head_stride / token_stride) + max_tokens;
-  } else {
-    return cudaErrorInvalidValue;
-  }
+  QkvCoords co;
   CUtensorMap tq, tk, tv;
-  if (!encode_2d_fp16_sw128(&tq, q, rows, cols, static_cast<uint64_t>(token_stride), kBoxRows, kD, maps) ||
-      !encode_2d_fp16_sw128(&tk, k, rows, cols, static_cast<uint64_t>(token_stride), kBoxRows, kD, maps) ||
-      !encode_2d_fp16_sw128(&tv, v, rows, cols, static_cast<uint64_t>(token_stride), kBoxRows, kD, maps))
+  if (!encode_qkv(q, k, v, token_stride, head_stride, heads, max_tokens, kBoxRows, kD, &co, &tq, &tk, &tv, maps))
     return cudaErrorInvalidValue;
   static PerDeviceOnce once;  // function attributes are per device
   const cudaError_t once_err = once.run([] {

@@ -212,10 +212,6 @@ __global__ void attention_plan_kernel(const int* cu_seqlens, const int* batch_id
   }
 }
 
-struct Coords {
-  int x_per_head, y_per_head;  // TMA coordinates: x = head * x_per_head, y = head * y_per_head + token
-};
-
 // General [B, S, S] attention mask (kMask kernels): attr_mask[b][q][k] > 0.5 = query position q of
 // sequence b may attend to key position k; batch_idx / word_idx give the sequence and the position of
 // every packed row.  Semantics of the reference op (cuda/attention.cu:106-382): the score of a
@@ -280,7 +276,7 @@ __device__ __forceinline__ void drain_attention(uint32_t bar_qk, uint32_t qk, ui
 template <bool kMask>
 __global__ void __launch_bounds__(kThreads, kCtasPerSm)
 attention_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_k,
-                         const __grid_constant__ CUtensorMap tmap_v, Coords co, __half* __restrict__ ctx,
+                         const __grid_constant__ CUtensorMap tmap_v, QkvCoords co, __half* __restrict__ ctx,
                          const int* plan, int batch, int max_tokens, int heads,
                          float scale_log2e, int* status_word, int reverse, MaskArgs ma) {
   // The prologue (barriers, TMEM) touches no global memory: it runs before the
@@ -639,7 +635,7 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_q, const __gri
 // balances that; those beyond a sequence's end leave at once.
 __global__ void __launch_bounds__(kThreads, kCtasPerSm)
 attention_tcgen05_long_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_k,
-                              const __grid_constant__ CUtensorMap tmap_v, Coords co, __half* __restrict__ ctx,
+                              const __grid_constant__ CUtensorMap tmap_v, QkvCoords co, __half* __restrict__ ctx,
                               const int* cu_seqlens, int max_tokens, int max_seq, int heads, int q_tiles,
                               float scale_log2e, int* status_word) {
   pdl_trigger();
@@ -871,24 +867,6 @@ attention_tcgen05_long_kernel(const __grid_constant__ CUtensorMap tmap_q, const 
   }
 }
 
-// How (token, head) maps to TMA coordinates, and the extent of the tensor they index.
-bool qkv_coords(long long token_stride, long long head_stride, int heads, int max_tokens, Coords* co, uint64_t* cols,
-                uint64_t* rows) {
-  if (static_cast<long long>(heads - 1) * head_stride + kD <= token_stride) {
-    *co = {static_cast<int>(head_stride), 0};
-    *cols = static_cast<uint64_t>(heads - 1) * head_stride + kD;
-    *rows = static_cast<uint64_t>(max_tokens);
-    return true;
-  }
-  if (token_stride == kD && head_stride % token_stride == 0 && head_stride / token_stride >= max_tokens) {
-    *co = {0, static_cast<int>(head_stride / token_stride)};
-    *cols = kD;
-    *rows = static_cast<uint64_t>(heads - 1) * (head_stride / token_stride) + max_tokens;
-    return true;
-  }
-  return false;
-}
-
 }  // namespace
 
 namespace {
@@ -905,6 +883,27 @@ cudaError_t launch_plan(const int* cu_seqlens, const int* batch_idx, const int* 
                     t_ptr, cu_out, batch, max_tokens, plan);
 }
 }  // namespace
+
+bool encode_qkv(const __half* q, const __half* k, const __half* v, long long token_stride, long long head_stride,
+                int heads, int max_tokens, uint32_t box_rows, uint32_t d, QkvCoords* co, CUtensorMap* tq,
+                CUtensorMap* tk, CUtensorMap* tv, TensorMapCache* maps) {
+  uint64_t cols, rows;
+  if (static_cast<long long>(heads - 1) * head_stride + d <= token_stride) {
+    *co = {static_cast<int>(head_stride), 0};
+    cols = static_cast<uint64_t>(heads - 1) * head_stride + d;
+    rows = static_cast<uint64_t>(max_tokens);
+  } else if (token_stride == d && head_stride % token_stride == 0 && head_stride / token_stride >= max_tokens) {
+    *co = {0, static_cast<int>(head_stride / token_stride)};
+    cols = d;
+    rows = static_cast<uint64_t>(heads - 1) * (head_stride / token_stride) + max_tokens;
+  } else {
+    return false;
+  }
+  const uint64_t stride = static_cast<uint64_t>(token_stride);
+  return encode_2d_fp16_sw128(tq, q, rows, cols, stride, box_rows, d, maps) &&
+         encode_2d_fp16_sw128(tk, k, rows, cols, stride, box_rows, d, maps) &&
+         encode_2d_fp16_sw128(tv, v, rows, cols, stride, box_rows, d, maps);
+}
 
 size_t attention_plan_ints(int batch, int max_tokens) { return plan_ints(batch, max_tokens); }
 
@@ -945,13 +944,9 @@ cudaError_t launch_attention_tcgen05(const __half* q, const __half* k, const __h
   if ((reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(k) | reinterpret_cast<uintptr_t>(v) |
        reinterpret_cast<uintptr_t>(ctx)) & 31u)
     return cudaErrorMisalignedAddress;
-  Coords co;
-  uint64_t cols, rows;
-  if (!qkv_coords(token_stride, head_stride, heads, max_tokens, &co, &cols, &rows)) return cudaErrorInvalidValue;
+  QkvCoords co;
   CUtensorMap tq, tk, tv;
-  if (!encode_2d_fp16_sw128(&tq, q, rows, cols, static_cast<uint64_t>(token_stride), kBoxRows, kD, maps) ||
-      !encode_2d_fp16_sw128(&tk, k, rows, cols, static_cast<uint64_t>(token_stride), kBoxRows, kD, maps) ||
-      !encode_2d_fp16_sw128(&tv, v, rows, cols, static_cast<uint64_t>(token_stride), kBoxRows, kD, maps))
+  if (!encode_qkv(q, k, v, token_stride, head_stride, heads, max_tokens, kBoxRows, kD, &co, &tq, &tk, &tv, maps))
     return cudaErrorInvalidValue;
   static PerDeviceOnce once;  // function attributes are per device
   const cudaError_t once_err = once.run([] {
@@ -994,13 +989,9 @@ cudaError_t launch_attention_tcgen05_long(const __half* q, const __half* k, cons
   if (((reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(k) | reinterpret_cast<uintptr_t>(v)) & 15u) ||
       (reinterpret_cast<uintptr_t>(ctx) & 31u))
     return cudaErrorMisalignedAddress;
-  Coords co;
-  uint64_t cols, rows;
-  if (!qkv_coords(token_stride, head_stride, heads, max_tokens, &co, &cols, &rows)) return cudaErrorInvalidValue;
+  QkvCoords co;
   CUtensorMap tq, tk, tv;
-  if (!encode_2d_fp16_sw128(&tq, q, rows, cols, static_cast<uint64_t>(token_stride), kBoxRows, kD, maps) ||
-      !encode_2d_fp16_sw128(&tk, k, rows, cols, static_cast<uint64_t>(token_stride), kBoxRows, kD, maps) ||
-      !encode_2d_fp16_sw128(&tv, v, rows, cols, static_cast<uint64_t>(token_stride), kBoxRows, kD, maps))
+  if (!encode_qkv(q, k, v, token_stride, head_stride, heads, max_tokens, kBoxRows, kD, &co, &tq, &tk, &tv, maps))
     return cudaErrorInvalidValue;
   static PerDeviceOnce once;  // function attributes are per device
   const cudaError_t once_err = once.run([] {

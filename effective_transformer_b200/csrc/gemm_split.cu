@@ -83,20 +83,6 @@ __device__ __forceinline__ float4 ld_shared_f4(uint32_t addr) {
 __device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
 __device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
 
-__device__ __forceinline__ uint32_t gelu_tanh_half2(uint32_t xbits) {  // as in gemm_tcgen05.cu
-  const __half2 x = *reinterpret_cast<const __half2*>(&xbits);
-  const __half2 c1 = __float2half2_rn(0.7978845608028654f);
-  const __half2 c2 = __float2half2_rn(0.7978845608028654f * 0.044715f);
-  const __half2 u = __hmul2(x, __hfma2(__hmul2(x, x), c2, c1));
-  const uint32_t ubits = *reinterpret_cast<const uint32_t*>(&u);
-  uint32_t tbits;
-  asm("tanh.approx.f16x2 %0, %1;" : "=r"(tbits) : "r"(ubits));
-  const __half2 th = *reinterpret_cast<const __half2*>(&tbits);
-  const __half2 hx = __hmul2(x, __float2half2_rn(0.5f));
-  const __half2 y = __hfma2(hx, th, hx);
-  return *reinterpret_cast<const uint32_t*>(&y);
-}
-
 __device__ __forceinline__ void load8(const __half* p, float* f) { VecTraits<__half>::unpack(ld_global_nc_v4(p), f); }
 __device__ __forceinline__ void load8(const float* p, float* f) {
   VecTraits<float>::unpack(ld_global_nc_v4(p), f);

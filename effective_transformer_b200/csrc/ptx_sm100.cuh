@@ -5,6 +5,7 @@
 #pragma once
 
 #include <cuda.h>
+#include <cuda_fp16.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
 
@@ -310,6 +311,15 @@ class TensorMapCache {
 bool encode_2d_fp16_sw128(CUtensorMap* map, const void* base, uint64_t rows, uint64_t cols,
                           uint64_t row_stride_elems, uint32_t box_rows, uint32_t box_cols,
                           TensorMapCache* cache = nullptr);
+// Q, K and V of the attention kernels, in either of two layouts: heads side by side inside a token row (x moves with
+// the head), or one [max_tokens, d] block per head (y moves with the head).
+struct QkvCoords {
+  int x_per_head, y_per_head;  // TMA coordinates: x = head * x_per_head, y = head * y_per_head + token
+};
+// Their tensor maps (box [box_rows, d]) and how (token, head) maps to coordinates; false for other strides.
+bool encode_qkv(const __half* q, const __half* k, const __half* v, long long token_stride, long long head_stride,
+                int heads, int max_tokens, uint32_t box_rows, uint32_t d, QkvCoords* co, CUtensorMap* tq,
+                CUtensorMap* tk, CUtensorMap* tv, TensorMapCache* maps);
 // fp32 row-major [rows, cols] tensor, box [box_rows, 32], 128-byte swizzle.
 bool encode_2d_f32_sw128(CUtensorMap* map, const void* base, uint64_t rows, uint64_t cols, uint32_t box_rows,
                          TensorMapCache* cache);
