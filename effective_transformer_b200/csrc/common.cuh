@@ -151,6 +151,21 @@ __device__ __forceinline__ Vec16 ld_activation_v4(const void* p) {
                : "memory");
   return v;
 }
+// The row count of a pass (*m_ptr, *t_ptr), from L2.  With `ready` it may be read in front of pdl_wait(): the kernel
+// that wrote it had completed before this kernel could be launched (see GemmHints).
+__device__ __forceinline__ int ld_row_count(const int* p) {
+  int v;
+  asm volatile("ld.relaxed.gpu.global.s32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+  return v;
+}
+// pdl_wait() and the row count, clamped to [0, max_rows]; a count that is ready comes in under the wait.
+__device__ __forceinline__ int pdl_wait_row_count(const int* p, int max_rows, int ready) {
+  int v = 0;
+  if (ready != 0) v = ld_row_count(p);
+  pdl_wait();
+  if (ready == 0) v = ld_row_count(p);
+  return v < 0 ? 0 : (v > max_rows ? max_rows : v);
+}
 // Through L2 only: for rows that other CTAs of the same kernel have just written.
 __device__ __forceinline__ Vec16 ld_global_cg_v4(const void* p) {
   Vec16 v;
@@ -286,13 +301,14 @@ cudaError_t launch_add_qkv_bias_transpose(const T* q, const T* bq, const T* k, c
 template <typename T>
 cudaError_t launch_add_bias_gelu(T* out, const T* bias, const int* t_ptr, int max_tokens, int n,
                                  cudaStream_t stream);
+// rows_ready: as in GemmHints.
 // split_hi / split_lo (fp32 only, both or neither): the normalised rows are also written as
 // rn_tf32 half and remainder, the input format of the fp32 projections on the tensor cores.
 template <typename T>
 cudaError_t launch_add_bias_input_layernorm(T* out, const T* input, const T* bias, const T* gamma,
                                             const T* beta, const int* t_ptr, int max_tokens, int n,
                                             float eps, cudaStream_t stream, bool reverse = false,
-                                            T* split_hi = nullptr, T* split_lo = nullptr);
+                                            T* split_hi = nullptr, T* split_lo = nullptr, bool rows_ready = false);
 // Embedding rows + LayerNorm for valid tokens only, written packed [T, n].
 // token_type_ids / type_table / pos_table may be null.
 template <typename T>
@@ -432,6 +448,19 @@ constexpr int kMaskBitsBytes = 32;  // per token
 cudaError_t launch_attention_mask_bits(const __half* attr_mask, const int* batch_idx, const int* word_idx,
                                        const int* cu_seqlens, const int* t_ptr, int max_tokens, int seq,
                                        uint32_t* bits, cudaStream_t stream);
+// What the caller of a projection knows about the stream it is launched into.
+struct GemmHints {
+  // w was complete before the preceding kernel of the stream began (the handle's own weights): a kernel may fetch it
+  // before it waits for that kernel.
+  bool weights_ready = false;
+  // So was *m_ptr before this kernel can be launched: the kernel that wrote it lies in front of one that lets its
+  // dependents start only behind its own pdl_wait() (the copy or embedding kernel behind the counting one; in the layer
+  // op the kernel that works out the sequence bounds).  The count is then read under the wait.
+  bool rows_ready = false;
+  // The capacity in rows by which the kernel is chosen, 0 = max_m.  The kernels round differently (order of the K sum,
+  // fp16 pairs or fp32 in an epilogue), so the parts of one batch name the whole batch's here.
+  int route_rows = 0;
+};
 // fp32 GEMM on the tensor cores by the three-product tf32 split (gemm_tf32x3.cu):
 // x = hi + lo with hi = rn_tf32(x); hi/lo may alias x.  rows_ptr null = max_rows.
 cudaError_t launch_split_tf32(const float* x, float* hi, float* lo, const int* rows_ptr, int max_rows, int cols,
@@ -441,22 +470,17 @@ cudaError_t launch_split_tf32(const float* x, float* hi, float* lo, const int* r
 cudaError_t launch_gemm_tf32x3(const float* a_hi, const float* a_lo, const float* w_hi, const float* w_lo,
                                const float* bias, float* c, const int* m_ptr, int max_m, int n, int k,
                                int epilogue, int* status_word, cudaStream_t stream, bool reverse_m = false,
-                               float* c_lo = nullptr, TensorMapCache* maps = nullptr, bool weights_ready = false,
-                               int route_rows = 0);
+                               float* c_lo = nullptr, TensorMapCache* maps = nullptr, GemmHints hints = GemmHints());
 // tcgen05 GEMM, fp16 in / fp32 accumulate / fp16 out.  w_packed is [N,K].
 // reverse_m: row tiles are visited from the last to the first.  A kernel that
 // consumes what the previous kernel has just written finds the rows written
 // last still in L2 if it starts with them, so consecutive kernels of a layer
 // alternate their direction.
-// weights_ready: w_packed was complete before the preceding kernel of the stream began (the handle's own
-// weights), so a kernel may fetch it before it waits for that kernel.
-// route_rows: the capacity in rows by which the kernel is chosen, 0 = max_m.  The kernels round differently (order
-// of the K sum, fp16 pairs or fp32 in an epilogue), so the parts of one batch name the whole batch's here.
 cudaError_t launch_gemm_tcgen05(const __half* a, const __half* w_packed, const __half* bias,
                                 __half* c, const int* m_ptr, int max_m, int n, int k, int epilogue,
                                 int* status_word, cudaStream_t stream, bool reverse_m = false,
                                 const __half* residual = nullptr, TensorMapCache* maps = nullptr,
-                                const GemmLayerNorm* ln = nullptr, bool weights_ready = false, int route_rows = 0);
+                                const GemmLayerNorm* ln = nullptr, GemmHints hints = GemmHints());
 // Projections of small batches on tiles of 128 x 64 (fp32 also 128 x 128) whose K range is split over a cluster
 // (gemm_split.cu).  fp16: a [max_m,k], w [n,k], c fp16.  a_lo / w_lo given: fp32 by the three-product tf32
 // split, c_lo as in launch_gemm_tf32x3.
@@ -471,7 +495,7 @@ struct SplitGemm {
   float* c_lo = nullptr;
   const int* m_ptr = nullptr;
   int max_m = 0, n = 0, k = 0;
-  bool weights_ready = false;  // w was complete before the preceding kernel of the stream began
+  GemmHints hints;
   int* status_word = nullptr;
   GemmLayerNorm ln;
 };

@@ -106,11 +106,10 @@ add_bias_input_layernorm_kernel(T* __restrict__ out, const T* input,
                                 const T* __restrict__ bias, const T* __restrict__ gamma,
                                 const T* __restrict__ beta, const int* t_ptr,
                                 int max_tokens, int n, float eps, int reverse, T* __restrict__ split_hi,
-                                T* __restrict__ split_lo) {
-  pdl_wait();
+                                T* __restrict__ split_lo, int rows_ready) {
+  const int t = pdl_wait_row_count(t_ptr, max_tokens, rows_ready);
   pdl_trigger();
   constexpr int E = VecTraits<T>::kElems;
-  const int t = clamp_tokens(t_ptr, max_tokens);
   const int lane = threadIdx.x & 31;
   const int warp = blockIdx.x * (kThreads / 32) + (threadIdx.x >> 5);
   const int nwarps = gridDim.x * (kThreads / 32);
@@ -323,7 +322,7 @@ template <typename T>
 cudaError_t launch_add_bias_input_layernorm(T* out, const T* input, const T* bias, const T* gamma,
                                             const T* beta, const int* t_ptr, int max_tokens, int n,
                                             float eps, cudaStream_t stream, bool reverse, T* split_hi,
-                                            T* split_lo) {
+                                            T* split_lo, bool rows_ready) {
   constexpr int E = VecTraits<T>::kElems;
   if (max_tokens <= 0) return cudaSuccess;
   if ((split_hi == nullptr) != (split_lo == nullptr) || (split_hi != nullptr && sizeof(T) != 4))
@@ -353,7 +352,8 @@ cudaError_t launch_add_bias_input_layernorm(T* out, const T* input, const T* bia
     const long long cap = static_cast<long long>(sm_count()) * per_sm;                                         \
     if (ctas > cap) ctas = cap;                                                                                \
     le = launch_pdl(kernel, dim3(static_cast<int>(ctas)), dim3(kThreads), 0, stream, out, input, bias, gamma,  \
-                    beta, t_ptr, max_tokens, n, eps, reverse ? 1 : 0, split_hi, split_lo);                     \
+                    beta, t_ptr, max_tokens, n, eps, reverse ? 1 : 0, split_hi, split_lo,   \
+                    rows_ready ? 1 : 0);                                                                                           \
   } while (0)
 #define ETB_LN(V, R_IN, R_NO)              \
   do {                                     \
@@ -396,7 +396,7 @@ cudaError_t launch_copy_columns(const T* src, T* dst, int rows, int cols, int ds
   template cudaError_t launch_add_bias_gelu<T>(T*, const T*, const int*, int, int, cudaStream_t); \
   template cudaError_t launch_add_bias_input_layernorm<T>(T*, const T*, const T*, const T*,      \
                                                           const T*, const int*, int, int, float, \
-                                                          cudaStream_t, bool, T*, T*);           \
+                                                          cudaStream_t, bool, T*, T*, bool);     \
   template cudaError_t launch_transpose<T>(const T*, T*, int, int, cudaStream_t);                \
   template cudaError_t launch_copy_columns<T>(const T*, T*, int, int, int, int, cudaStream_t);
 ETB_INST(float)

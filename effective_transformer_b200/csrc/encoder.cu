@@ -221,6 +221,14 @@ struct et_handle_s {
   // Rows by which the projections' kernels are chosen, 0 = the pass's own capacity.  A host-buffer call sets the
   // whole batch's for the passes over its chunks: their shares follow measured times, the result must not.
   int route_rows = 0;
+  // The layers' projections: packed weights, and a token count that the pass (or the caller of the layer op) had
+  // before the kernel in front of the first layer started.
+  GemmHints hints() const {
+    GemmHints g;
+    g.weights_ready = g.rows_ready = true;
+    g.route_rows = route_rows;
+    return g;
+  }
   std::vector<LayerWeights> layers;
   ModelWeights model;
   Workspace ws;
@@ -497,8 +505,7 @@ int run_layer(et_handle_t h, const LayerWeights& lw, const T* x_in, T* x_out, co
     if (tc)
       return launch_gemm_tcgen05(reinterpret_cast<const __half*>(a), static_cast<const __half*>(w_t),
                                  static_cast<const __half*>(bias), reinterpret_cast<__half*>(c), t_ptr,
-                                 max_m, n, k, epi, ws.status, s, turn(), nullptr, &h->maps, nullptr, true,
-                                 h->route_rows);
+                                 max_m, n, k, epi, ws.status, s, turn(), nullptr, &h->maps, nullptr, h->hints());
     if (tc32) {
       // w_t holds rn_tf32(W), w_lo the remainder; the input is split the same way first
       const float* a_hi = reinterpret_cast<const float*>(a);
@@ -511,7 +518,7 @@ int run_layer(et_handle_t h, const LayerWeights& lw, const T* x_in, T* x_out, co
       }
       return launch_gemm_tf32x3(a_hi, a_lo, static_cast<const float*>(w_t), static_cast<const float*>(w_lo),
                                 static_cast<const float*>(bias), reinterpret_cast<float*>(c), t_ptr, max_m, n, k,
-                                epi, ws.status, s, turn(), c_lo, &h->maps, true, h->route_rows);
+                                epi, ws.status, s, turn(), c_lo, &h->maps, h->hints());
     }
     forward_only();
     return launch_gemm_simt<T>(a, B(w_rm), B(bias), c, t_ptr, max_m, n, k, epi, s);
@@ -534,8 +541,8 @@ int run_layer(et_handle_t h, const LayerWeights& lw, const T* x_in, T* x_out, co
     nin.csum = H16(lw.cqkv);
     ET_LAUNCH(h, ET_PROF_GEMM_QKV, 1, s,
               launch_gemm_tcgen05(H16(x_in), H16(lw.wqkv_f), H16(lw.bqkv_f), reinterpret_cast<__half*>(qkv), t_ptr,
-                                  max_m, 3 * hid, hid, kEpiNormIn, ws.status, s, turn(), nullptr, &h->maps, &nin, true,
-                                  h->route_rows));
+                                  max_m, 3 * hid, hid, kEpiNormIn, ws.status, s, turn(), nullptr, &h->maps, &nin,
+                                  h->hints()));
   } else if (tc32 && in_split_ready)
     ET_LAUNCH(h, ET_PROF_GEMM_QKV, 1, s,
               gemm(reinterpret_cast<const T*>(ws.a_hi), lw.wqkv, lw.wqkv_t, lw.wqkv_lo, lw.bqkv, qkv, 3 * hid, hid,
@@ -600,8 +607,8 @@ int run_layer(et_handle_t h, const LayerWeights& lw, const T* x_in, T* x_out, co
     n1.stats_out = ws.stats_att;
     ET_LAUNCH(h, ET_PROF_GEMM_ATTN_OUT, 1, s,
               launch_gemm_tcgen05(H16(ctx), H16(lw.wo_t), H16(lw.bo), reinterpret_cast<__half*>(att), t_ptr, max_m,
-                                  hid, hid, kEpiNormResidual, ws.status, s, turn(), H16(x_in), &h->maps, &n1, true,
-                                  h->route_rows));
+                                  hid, hid, kEpiNormResidual, ws.status, s, turn(), H16(x_in), &h->maps, &n1,
+                                  h->hints()));
     // first feed-forward projection of LN1(att): folded weights, statistics, GELU
     GemmLayerNorm n2;
     n2.eps = h->eps;
@@ -610,7 +617,8 @@ int run_layer(et_handle_t h, const LayerWeights& lw, const T* x_in, T* x_out, co
     n2.csum = H16(lw.c1);
     ET_LAUNCH(h, ET_PROF_GEMM_FFN1, 1, s,
               launch_gemm_tcgen05(H16(att), H16(lw.w1_f), H16(lw.b1_f), reinterpret_cast<__half*>(ffn), t_ptr, max_m,
-                                  f, hid, kEpiNormInGelu, ws.status, s, turn(), nullptr, &h->maps, &n2, true, h->route_rows));
+                                  f, hid, kEpiNormInGelu, ws.status, s, turn(), nullptr, &h->maps, &n2,
+                                  h->hints()));
     // second: + bias + LN1(att) on the fly; leaves the sum in x_out and its statistics in ws.stats_x
     GemmLayerNorm n3;
     n3.eps = h->eps;
@@ -621,7 +629,8 @@ int run_layer(et_handle_t h, const LayerWeights& lw, const T* x_in, T* x_out, co
     n3.stats_out = ws.stats_x;
     ET_LAUNCH(h, ET_PROF_GEMM_FFN2, 1, s,
               launch_gemm_tcgen05(H16(ffn), H16(lw.w2_t), H16(lw.b2), reinterpret_cast<__half*>(x_out), t_ptr, max_m,
-                                  hid, f, kEpiNormResidual, ws.status, s, turn(), H16(att), &h->maps, &n3, true, h->route_rows));
+                                  hid, f, kEpiNormResidual, ws.status, s, turn(), H16(att), &h->maps, &n3,
+                                  h->hints()));
     return ET_OK;
   }
   const bool ln_in_gemm = tc && h->fuse_ln && gemm_layernorm_supported(hid);
@@ -644,7 +653,7 @@ int run_layer(et_handle_t h, const LayerWeights& lw, const T* x_in, T* x_out, co
                    reinterpret_cast<const float*>(ctx_lo)));
     ET_LAUNCH(h, ET_PROF_LAYERNORM, 1, s,
               launch_add_bias_input_layernorm<T>(att, x_in, B(lw.bo), B(lw.ln1_gamma), B(lw.ln1_beta), t_ptr, max_m,
-                                                 hid, h->eps, s, turn(), ln_hi, ln_lo));
+                                                 hid, h->eps, s, turn(), ln_hi, ln_lo, true));
   }
   // feed-forward: bias + GELU fused into the first GEMM
   // (fp32 tensor path: the GELU output leaves the epilogue split for the second projection)
@@ -664,18 +673,18 @@ int run_layer(et_handle_t h, const LayerWeights& lw, const T* x_in, T* x_out, co
   } else if (tc) {
     ET_LAUNCH(h, ET_PROF_GEMM_FFN2, 1, s,
               launch_gemm_tcgen05(H16(ffn), H16(lw.w2_t), H16(lw.b2), reinterpret_cast<__half*>(x_out), t_ptr, max_m,
-                                  hid, f, kEpiBiasResidual, ws.status, s, turn(), H16(att), &h->maps, nullptr, true,
-                                  h->route_rows));
+                                  hid, f, kEpiBiasResidual, ws.status, s, turn(), H16(att), &h->maps, nullptr,
+                                  h->hints()));
     ET_LAUNCH(h, ET_PROF_LAYERNORM, 1, s,
               launch_add_bias_input_layernorm<T>(x_out, nullptr, nullptr, B(lw.ln2_gamma), B(lw.ln2_beta), t_ptr,
-                                                 max_m, hid, h->eps, s, turn()));
+                                                 max_m, hid, h->eps, s, turn(), nullptr, nullptr, true));
   } else {
     ET_LAUNCH(h, ET_PROF_GEMM_FFN2, 1, s,
               gemm(ffn, lw.w2, lw.w2_t, lw.w2_lo, nullptr, x_out, hid, f, kEpiNone, tc32 ? ws.ffn_lo : nullptr));
     const bool split2 = tc32 && out_split;
     ET_LAUNCH(h, ET_PROF_LAYERNORM, 1, s, launch_add_bias_input_layernorm<T>(x_out, att, B(lw.b2), B(lw.ln2_gamma), B(lw.ln2_beta),
                                                   t_ptr, max_m, hid, h->eps, s, turn(), split2 ? ln_hi : nullptr,
-                                                  split2 ? ln_lo : nullptr));
+                                                  split2 ? ln_lo : nullptr, true));
   }
   return ET_OK;
 }
@@ -815,7 +824,7 @@ int stack_impl(et_handle_t h, int batch, int seq, cudaStream_t s) {
               launch_add_bias_input_layernorm<__half>(static_cast<__half*>(ws.x), nullptr, nullptr,
                                                       static_cast<const __half*>(last.ln2_gamma),
                                                       static_cast<const __half*>(last.ln2_beta), ws.valid_word_num,
-                                                      max_m, h->hidden, h->eps, s, reverse));
+                                                      max_m, h->hidden, h->eps, s, reverse, nullptr, nullptr, true));
   }
   return ET_OK;
 }
@@ -846,6 +855,8 @@ int pooler_impl(et_handle_t h, const void* packed, const int* cu_seqlens, void* 
   Workspace& ws = h->ws;
   const ModelWeights& mw = h->model;
   const int hid = h->hidden;
+  GemmHints pool_hints;  // (the row count comes from the kernel in front)
+  pool_hints.weights_ready = true;
   ET_LAUNCH(h, ET_PROF_POOLER, 1, s,
             launch_gather_first_tokens(packed, cu_seqlens, ws.first_tok, batch, max_tokens,
                                        hid * static_cast<int>(h->esize), ws.pool_m, s));
@@ -853,7 +864,8 @@ int pooler_impl(et_handle_t h, const void* packed, const int* cu_seqlens, void* 
     ET_LAUNCH(h, ET_PROF_POOLER, 1, s,
               launch_gemm_tcgen05(static_cast<const __half*>(ws.first_tok), static_cast<const __half*>(mw.pool_w_t),
                                   static_cast<const __half*>(mw.pool_b), static_cast<__half*>(pooled_out),
-                                  ws.pool_m, batch, hid, hid, kEpiBiasTanh, ws.status, s, false, nullptr, &h->maps, nullptr, true));
+                                  ws.pool_m, batch, hid, hid, kEpiBiasTanh, ws.status, s, false, nullptr, &h->maps, nullptr,
+                                  pool_hints));
   else if (h->cfg.dtype == ET_FP16)
     ET_LAUNCH(h, ET_PROF_POOLER, 1, s,
               launch_gemm_simt<__half>(static_cast<const __half*>(ws.first_tok), static_cast<const __half*>(mw.pool_w),

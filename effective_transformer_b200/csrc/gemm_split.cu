@@ -150,7 +150,7 @@ gemm_split_kernel(const __grid_constant__ Maps maps, void* __restrict__ c_ptr, f
     *abort_flag = 1;
     report_timeout(status_word, kKernelGemmTc, 16 + site);
   };
-  auto valid_rows = [&]() {
+  auto valid_rows = [&]() {  // behind pdl_wait()
     const int M = *m_ptr;
     return (M < 0 ? 0 : (M > max_m ? max_m : M)) - m0;  // of this tile, <= 0: nothing to do
   };
@@ -501,7 +501,7 @@ cudaError_t launch_split_bn(const Maps& maps, const SplitGemm& g, int splits, cu
   lc.attrs = attr;
   lc.numAttrs = pdl_enabled() ? 2 : 1;
   return cudaLaunchKernelEx(&lc, gemm_split_kernel<kTf32, BN, EPI>, maps, g.c, g.c_lo, g.bias, g.residual, g.m_ptr,
-                            g.max_m, g.n, (g.k + cfg::BK - 1) / cfg::BK, g.weights_ready ? 1 : 0, g.status_word, g.ln);
+                            g.max_m, g.n, (g.k + cfg::BK - 1) / cfg::BK, g.hints.weights_ready ? 1 : 0, g.status_word, g.ln);
 }
 
 template <bool kTf32, int EPI>

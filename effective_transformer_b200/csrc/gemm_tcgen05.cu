@@ -399,7 +399,7 @@ __global__ void __launch_bounds__(kNumThreads, 1)
 gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a,
                     const __grid_constant__ CUtensorMap tmap_b, __half* __restrict__ C,
                     const __half* __restrict__ bias, const __half* residual,
-                    const int* m_ptr, int max_m, int N, int K, int* status_word, int reverse_m) {
+                    const int* m_ptr, int max_m, int N, int K, int* status_word, int reverse_m, int rows_ready) {
   using cfg = Cfg<BN>;
   constexpr int S = cfg::kStages;
 
@@ -452,9 +452,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a,
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
 
-  pdl_wait();  // M and the A rows come from earlier kernels
-  int M = *m_ptr;
-  M = M < 0 ? 0 : (M > max_m ? max_m : M);
+  const int M = pdl_wait_row_count(m_ptr, max_m, rows_ready);  // M and the A rows come from earlier kernels
   const int m_tiles = (M + BM - 1) / BM;
   const int n_tiles = N / BN;
   const int num_tiles = m_tiles * n_tiles;  // 0: every role's loop is empty
@@ -650,7 +648,7 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap tmap_a,
                          const __grid_constant__ CUtensorMap tmap_b_half, __half* __restrict__ C,
                          const __half* __restrict__ bias, const __half* residual,
                          const int* m_ptr, int max_m, int N, int K, int* status_word,
-                         int reverse_m, const GemmLayerNorm ln) {
+                         int reverse_m, int rows_ready, const GemmLayerNorm ln) {
   using cfg = PairCfg;
   constexpr int S = cfg::kStages;
   constexpr int BN = cfg::BN;
@@ -718,9 +716,7 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap tmap_a,
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
 
-  pdl_wait();  // M and the A rows come from earlier kernels
-  int M = *m_ptr;
-  M = M < 0 ? 0 : (M > max_m ? max_m : M);
+  const int M = pdl_wait_row_count(m_ptr, max_m, rows_ready);  // M and the A rows come from earlier kernels
   const int m_tiles = (M + BM2 - 1) / BM2;
   const int n_tiles = N / BN;
   const int num_tiles = m_tiles * n_tiles;  // 0: every role's loop is empty
@@ -1127,7 +1123,7 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap tmap_a,
 template <int EPI, int VPL>
 cudaError_t launch_pair_epi(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& tbh,
                             const __half* bias, const __half* residual, __half* c,
-                            const int* m_ptr, int max_m, int n, int k, int* status_word, int reverse_m,
+                            const int* m_ptr, int max_m, int n, int k, int* status_word, int reverse_m, int rows_ready,
                             const GemmLayerNorm& ln, cudaStream_t stream) {
   using cfg = PairCfg;
   static PerDeviceOnce once;  // function attributes are per device
@@ -1143,7 +1139,7 @@ cudaError_t launch_pair_epi(const CUtensorMap& ta, const CUtensorMap& tb, const 
   if (pairs > 2 * max_tiles) pairs = 2 * max_tiles;
   if (pairs < 1) pairs = 1;
   return launch_pdl(gemm_tcgen05_pair_kernel<EPI, VPL>, dim3(static_cast<int>(2 * pairs)), dim3(threads_of(EPI)),
-                    cfg::kSmemBytes, stream, ta, tb, tbh, c, bias, residual, m_ptr, max_m, n, k, status_word, reverse_m,
+                    cfg::kSmemBytes, stream, ta, tb, tbh, c, bias, residual, m_ptr, max_m, n, k, status_word, reverse_m, rows_ready,
                     ln);
 }
 
@@ -1151,11 +1147,11 @@ cudaError_t launch_pair_epi(const CUtensorMap& ta, const CUtensorMap& tb, const 
 template <int EPI>
 cudaError_t launch_pair_ln(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& tbh,
                            const __half* bias, const __half* residual, __half* c, const int* m_ptr, int max_m,
-                           int n, int k, int* status_word, int reverse_m, const GemmLayerNorm& ln,
+                           int n, int k, int* status_word, int reverse_m, int rows_ready, const GemmLayerNorm& ln,
                            cudaStream_t stream) {
 #define ETB_LN_CASE(V)                                                                                            \
   case V:                                                                                                         \
-    return launch_pair_epi<EPI, V>(ta, tb, tbh, bias, residual, c, m_ptr, max_m, n, k, status_word, reverse_m, ln, \
+    return launch_pair_epi<EPI, V>(ta, tb, tbh, bias, residual, c, m_ptr, max_m, n, k, status_word, reverse_m, rows_ready, ln, \
                                    stream)
   switch (n >> 8) {
     ETB_LN_CASE(1);
@@ -1173,11 +1169,11 @@ cudaError_t launch_pair_ln(const CUtensorMap& ta, const CUtensorMap& tb, const C
 template <int EPI>
 cudaError_t launch_pair_norm(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& tbh,
                              const __half* bias, const __half* residual, __half* c, const int* m_ptr, int max_m,
-                             int n, int k, int* status_word, int reverse_m, const GemmLayerNorm& ln,
+                             int n, int k, int* status_word, int reverse_m, int rows_ready, const GemmLayerNorm& ln,
                              cudaStream_t stream) {
 #define ETB_NORM_CASE(V)                                                                                          \
   case V:                                                                                                         \
-    return launch_pair_epi<EPI, V>(ta, tb, tbh, bias, residual, c, m_ptr, max_m, n, k, status_word, reverse_m, ln, \
+    return launch_pair_epi<EPI, V>(ta, tb, tbh, bias, residual, c, m_ptr, max_m, n, k, status_word, reverse_m, rows_ready, ln, \
                                    stream)
   const int width = EPI == kEpiNormResidual ? n : k;
   switch (width / 128) {
@@ -1194,10 +1190,10 @@ cudaError_t launch_pair_norm(const CUtensorMap& ta, const CUtensorMap& tb, const
 cudaError_t launch_pair(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& tbh,
                         const __half* bias, const __half* residual, __half* c,
                         const int* m_ptr, int max_m, int n, int k, int epilogue, int* status_word,
-                        int reverse_m, const GemmLayerNorm& ln, cudaStream_t stream) {
+                        int reverse_m, int rows_ready, const GemmLayerNorm& ln, cudaStream_t stream) {
 #define ETB_PAIR_CASE(E)                                                                                      \
   case E:                                                                                                     \
-    return launch_pair_epi<E, 0>(ta, tb, tbh, bias, residual, c, m_ptr, max_m, n, k, status_word, reverse_m, ln, \
+    return launch_pair_epi<E, 0>(ta, tb, tbh, bias, residual, c, m_ptr, max_m, n, k, status_word, reverse_m, rows_ready, ln, \
                                  stream)
   switch (epilogue) {
     ETB_PAIR_CASE(kEpiNone);
@@ -1206,20 +1202,20 @@ cudaError_t launch_pair(const CUtensorMap& ta, const CUtensorMap& tb, const CUte
     ETB_PAIR_CASE(kEpiBiasTanh);
     ETB_PAIR_CASE(kEpiBiasResidual);
     case kEpiNormIn:
-      return launch_pair_norm<kEpiNormIn>(ta, tb, tbh, bias, residual, c, m_ptr, max_m, n, k, status_word, reverse_m,
+      return launch_pair_norm<kEpiNormIn>(ta, tb, tbh, bias, residual, c, m_ptr, max_m, n, k, status_word, reverse_m, rows_ready,
                                           ln, stream);
     case kEpiNormInGelu:
       return launch_pair_norm<kEpiNormInGelu>(ta, tb, tbh, bias, residual, c, m_ptr, max_m, n, k, status_word,
-                                              reverse_m, ln, stream);
+                                              reverse_m, rows_ready, ln, stream);
     case kEpiNormResidual:
       return launch_pair_norm<kEpiNormResidual>(ta, tb, tbh, bias, residual, c, m_ptr, max_m, n, k, status_word,
-                                                reverse_m, ln, stream);
+                                                reverse_m, rows_ready, ln, stream);
     case kEpiResidualLayerNorm:
       return launch_pair_ln<kEpiResidualLayerNorm>(ta, tb, tbh, bias, residual, c, m_ptr, max_m, n, k, status_word,
-                                                   reverse_m, ln, stream);
+                                                   reverse_m, rows_ready, ln, stream);
     case kEpiLayerNorm:
       return launch_pair_ln<kEpiLayerNorm>(ta, tb, tbh, bias, residual, c, m_ptr, max_m, n, k, status_word,
-                                           reverse_m, ln, stream);
+                                           reverse_m, rows_ready, ln, stream);
     default:
       return cudaErrorInvalidValue;
   }
@@ -1228,7 +1224,7 @@ cudaError_t launch_pair(const CUtensorMap& ta, const CUtensorMap& tb, const CUte
 
 template <int BN, int EPI>
 cudaError_t launch_bn_epi(const CUtensorMap& ta, const CUtensorMap& tb, const __half* bias, const __half* residual, __half* c,
-                          const int* m_ptr, int max_m, int n, int k, int* status_word, int reverse_m,
+                          const int* m_ptr, int max_m, int n, int k, int* status_word, int reverse_m, int rows_ready,
                           cudaStream_t stream) {
   using cfg = Cfg<BN>;
   static PerDeviceOnce once;  // function attributes are per device
@@ -1243,25 +1239,25 @@ cudaError_t launch_bn_epi(const CUtensorMap& ta, const CUtensorMap& tb, const __
   if (grid > max_tiles) grid = max_tiles;
   if (grid < 1) grid = 1;
   return launch_pdl(gemm_tcgen05_kernel<BN, EPI>, dim3(static_cast<int>(grid)), dim3(kNumThreads),
-                    cfg::kSmemBytes, stream, ta, tb, c, bias, residual, m_ptr, max_m, n, k, status_word, reverse_m);
+                    cfg::kSmemBytes, stream, ta, tb, c, bias, residual, m_ptr, max_m, n, k, status_word, reverse_m, rows_ready);
 }
 
 template <int BN>
 cudaError_t launch_bn(const CUtensorMap& ta, const CUtensorMap& tb, const __half* bias, const __half* residual, __half* c,
                       const int* m_ptr, int max_m, int n, int k, int epilogue, int* status_word,
-                      int reverse_m, cudaStream_t stream) {
+                      int reverse_m, int rows_ready, cudaStream_t stream) {
   switch (epilogue) {
     case kEpiNone:
-      return launch_bn_epi<BN, kEpiNone>(ta, tb, bias, residual, c, m_ptr, max_m, n, k, status_word, reverse_m, stream);
+      return launch_bn_epi<BN, kEpiNone>(ta, tb, bias, residual, c, m_ptr, max_m, n, k, status_word, reverse_m, rows_ready, stream);
     case kEpiBias:
-      return launch_bn_epi<BN, kEpiBias>(ta, tb, bias, residual, c, m_ptr, max_m, n, k, status_word, reverse_m, stream);
+      return launch_bn_epi<BN, kEpiBias>(ta, tb, bias, residual, c, m_ptr, max_m, n, k, status_word, reverse_m, rows_ready, stream);
     case kEpiBiasGelu:
-      return launch_bn_epi<BN, kEpiBiasGelu>(ta, tb, bias, residual, c, m_ptr, max_m, n, k, status_word, reverse_m, stream);
+      return launch_bn_epi<BN, kEpiBiasGelu>(ta, tb, bias, residual, c, m_ptr, max_m, n, k, status_word, reverse_m, rows_ready, stream);
     case kEpiBiasTanh:
-      return launch_bn_epi<BN, kEpiBiasTanh>(ta, tb, bias, residual, c, m_ptr, max_m, n, k, status_word, reverse_m, stream);
+      return launch_bn_epi<BN, kEpiBiasTanh>(ta, tb, bias, residual, c, m_ptr, max_m, n, k, status_word, reverse_m, rows_ready, stream);
     case kEpiBiasResidual:
       return launch_bn_epi<BN, kEpiBiasResidual>(ta, tb, bias, residual, c, m_ptr, max_m, n, k, status_word,
-                                                 reverse_m, stream);
+                                                 reverse_m, rows_ready, stream);
     default:
       return cudaErrorInvalidValue;
   }
@@ -1321,7 +1317,7 @@ bool encode_2d_fp16_sw128(CUtensorMap* map, const void* base, uint64_t rows, uin
 cudaError_t launch_gemm_tcgen05(const __half* a, const __half* w_packed, const __half* bias,
                                 __half* c, const int* m_ptr, int max_m, int n, int k, int epilogue,
                                 int* status_word, cudaStream_t stream, bool reverse_m, const __half* residual,
-                                TensorMapCache* maps, const GemmLayerNorm* ln, bool weights_ready, int route_rows) {
+                                TensorMapCache* maps, const GemmLayerNorm* ln, GemmHints hints) {
   if (max_m <= 0) return cudaSuccess;
   if (n <= 0 || k <= 0 || (n % 128) != 0 || (k % 8) != 0) return cudaErrorInvalidValue;
   if ((reinterpret_cast<uintptr_t>(a) & 15u) || (reinterpret_cast<uintptr_t>(w_packed) & 15u) ||
@@ -1360,11 +1356,11 @@ cudaError_t launch_gemm_tcgen05(const __half* a, const __half* w_packed, const _
     }
     lnp = *ln;
   }
-  if (const SplitPlan plan = gemm_route(false, route_rows > 0 ? route_rows : max_m, n, k, epilogue); plan.splits != 0) {
+  if (const SplitPlan plan = gemm_route(false, hints.route_rows > 0 ? hints.route_rows : max_m, n, k, epilogue); plan.splits != 0) {
     SplitGemm g;
     g.a = a, g.w = w_packed, g.bias = bias, g.residual = residual, g.c = c;
     g.m_ptr = m_ptr, g.max_m = max_m, g.n = n, g.k = k;
-    g.weights_ready = weights_ready;
+    g.hints = hints;
     g.status_word = status_word;
     g.ln = lnp;
     return launch_gemm_split(g, epilogue, plan, maps, stream);
@@ -1378,15 +1374,15 @@ cudaError_t launch_gemm_tcgen05(const __half* a, const __half* w_packed, const _
   if (!encode_2d_fp16_sw128(&tb, w_packed, static_cast<uint64_t>(n), static_cast<uint64_t>(k),
                             static_cast<uint64_t>(k), static_cast<uint32_t>(pair ? 128 : bn), BK, maps))
     return cudaErrorInvalidValue;
-  const int rev = reverse_m ? 1 : 0;
+  const int rev = reverse_m ? 1 : 0, rows_ready = hints.rows_ready ? 1 : 0;
   if (pair) {
     CUtensorMap tbh;  // 64 W rows per CTA: the half-width units of the last round
     if (!encode_2d_fp16_sw128(&tbh, w_packed, static_cast<uint64_t>(n), static_cast<uint64_t>(k),
                               static_cast<uint64_t>(k), 64, BK, maps))
       return cudaErrorInvalidValue;
-    return launch_pair(ta, tb, tbh, bias, residual, c, m_ptr, max_m, n, k, epilogue, status_word, rev, lnp, stream);
+    return launch_pair(ta, tb, tbh, bias, residual, c, m_ptr, max_m, n, k, epilogue, status_word, rev, rows_ready, lnp, stream);
   }
-  return launch_bn<128>(ta, tb, bias, residual, c, m_ptr, max_m, n, k, epilogue, status_word, rev, stream);
+  return launch_bn<128>(ta, tb, bias, residual, c, m_ptr, max_m, n, k, epilogue, status_word, rev, rows_ready, stream);
 }
 
 }  // namespace etb

@@ -228,7 +228,7 @@ __global__ void __launch_bounds__(kNumThreads, 1)
 gemm_tf32x3_kernel(const __grid_constant__ CUtensorMap tmap_a_hi, const __grid_constant__ CUtensorMap tmap_a_lo,
                    const __grid_constant__ CUtensorMap tmap_w_hi, const __grid_constant__ CUtensorMap tmap_w_lo,
                    float* __restrict__ C, float* __restrict__ c_lo, const float* __restrict__ bias,
-                   const int* m_ptr, int max_m, int N, int K, int* status_word, int reverse_m) {
+                   const int* m_ptr, int max_m, int N, int K, int* status_word, int reverse_m, int rows_ready) {
   using cfg = Cfg;
   constexpr int S = cfg::kStages;
 
@@ -278,9 +278,7 @@ gemm_tf32x3_kernel(const __grid_constant__ CUtensorMap tmap_a_hi, const __grid_c
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
 
-  pdl_wait();  // M and the A rows come from earlier kernels
-  int M = *m_ptr;
-  M = M < 0 ? 0 : (M > max_m ? max_m : M);
+  const int M = pdl_wait_row_count(m_ptr, max_m, rows_ready);  // M and the A rows come from earlier kernels
   const int m_tiles = (M + BM - 1) / BM;
   const int n_tiles = N / BN;
   const int num_tiles = m_tiles * n_tiles;  // 0: every role's loop is empty
@@ -500,7 +498,7 @@ gemm_tf32x3_pair_kernel(const __grid_constant__ CUtensorMap tmap_a_hi, const __g
                         const __grid_constant__ CUtensorMap tmap_w_hi_half,
                         const __grid_constant__ CUtensorMap tmap_w_lo_half, float* __restrict__ C,
                         float* __restrict__ c_lo, const float* __restrict__ bias, const int* m_ptr,
-                        int max_m, int N, int K, int* status_word, int reverse_m) {
+                        int max_m, int N, int K, int* status_word, int reverse_m, int rows_ready) {
   using cfg = PairCfg;
   constexpr int S = cfg::kStages;
 
@@ -552,9 +550,7 @@ gemm_tf32x3_pair_kernel(const __grid_constant__ CUtensorMap tmap_a_hi, const __g
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
 
-  pdl_wait();  // M and the A rows come from earlier kernels
-  int M = *m_ptr;
-  M = M < 0 ? 0 : (M > max_m ? max_m : M);
+  const int M = pdl_wait_row_count(m_ptr, max_m, rows_ready);  // M and the A rows come from earlier kernels
   const int m_tiles = (M + BM2 - 1) / BM2;
   const int n_tiles = N / BN2;
   const int num_tiles = m_tiles * n_tiles;  // 0: every role's loop is empty
@@ -748,7 +744,7 @@ gemm_tf32x3_pair_kernel(const __grid_constant__ CUtensorMap tmap_a_hi, const __g
 template <int EPI>
 cudaError_t launch_epi(const CUtensorMap& tah, const CUtensorMap& tal, const CUtensorMap& twh, const CUtensorMap& twl,
                        const float* bias, float* c, float* c_lo, const int* m_ptr, int max_m, int n, int k,
-                       int* status_word, int reverse_m, cudaStream_t stream) {
+                       int* status_word, int reverse_m, int rows_ready, cudaStream_t stream) {
   static PerDeviceOnce once;  // function attributes are per device
   const cudaError_t once_err = once.run([] {
     cudaError_t attr_err = cudaFuncSetAttribute(gemm_tf32x3_kernel<EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -761,14 +757,14 @@ cudaError_t launch_epi(const CUtensorMap& tah, const CUtensorMap& tal, const CUt
   if (grid > max_tiles) grid = max_tiles;
   if (grid < 1) grid = 1;
   return launch_pdl(gemm_tf32x3_kernel<EPI>, dim3(static_cast<int>(grid)), dim3(kNumThreads), Cfg::kSmemBytes, stream,
-                    tah, tal, twh, twl, c, c_lo, bias, m_ptr, max_m, n, k, status_word, reverse_m);
+                    tah, tal, twh, twl, c, c_lo, bias, m_ptr, max_m, n, k, status_word, reverse_m, rows_ready);
 }
 
 template <int EPI>
 cudaError_t launch_pair_epi(const CUtensorMap& tah, const CUtensorMap& tal, const CUtensorMap& twh,
                             const CUtensorMap& twl, const CUtensorMap& twhh, const CUtensorMap& twlh, const float* bias,
                             float* c, float* c_lo, const int* m_ptr, int max_m, int n, int k, int* status_word,
-                            int reverse_m, cudaStream_t stream) {
+                            int reverse_m, int rows_ready, cudaStream_t stream) {
   static PerDeviceOnce once;  // function attributes are per device
   const cudaError_t once_err = once.run([] {
     cudaError_t attr_err = cudaFuncSetAttribute(gemm_tf32x3_pair_kernel<EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -782,7 +778,7 @@ cudaError_t launch_pair_epi(const CUtensorMap& tah, const CUtensorMap& tal, cons
   if (pairs < 1) pairs = 1;
   return launch_pdl(gemm_tf32x3_pair_kernel<EPI>, dim3(static_cast<int>(2 * pairs)), dim3(kPairThreads),
                     PairCfg::kSmemBytes, stream, tah, tal, twh, twl, twhh, twlh, c, c_lo, bias, m_ptr, max_m, n, k,
-                    status_word, reverse_m);
+                    status_word, reverse_m, rows_ready);
 }
 
 }  // namespace
@@ -824,7 +820,7 @@ cudaError_t launch_split_tf32(const float* x, float* hi, float* lo, const int* r
 cudaError_t launch_gemm_tf32x3(const float* a_hi, const float* a_lo, const float* w_hi, const float* w_lo,
                                const float* bias, float* c, const int* m_ptr, int max_m, int n, int k,
                                int epilogue, int* status_word, cudaStream_t stream, bool reverse_m, float* c_lo,
-                               TensorMapCache* maps, bool weights_ready, int route_rows) {
+                               TensorMapCache* maps, GemmHints hints) {
   if (max_m <= 0) return cudaSuccess;
   if (n <= 0 || k <= 0 || (n % 128) != 0 || (k % BK) != 0) return cudaErrorInvalidValue;
   for (const void* p : {static_cast<const void*>(a_hi), static_cast<const void*>(a_lo),
@@ -834,11 +830,11 @@ cudaError_t launch_gemm_tf32x3(const float* a_hi, const float* a_lo, const float
   if (bias != nullptr && (reinterpret_cast<uintptr_t>(bias) & 15u)) return cudaErrorMisalignedAddress;
   if (c_lo != nullptr && (reinterpret_cast<uintptr_t>(c_lo) & 15u)) return cudaErrorMisalignedAddress;
   if (epilogue != kEpiNone && bias == nullptr) return cudaErrorInvalidValue;
-  if (const SplitPlan plan = gemm_route(true, route_rows > 0 ? route_rows : max_m, n, k, epilogue); plan.splits != 0) {
+  if (const SplitPlan plan = gemm_route(true, hints.route_rows > 0 ? hints.route_rows : max_m, n, k, epilogue); plan.splits != 0) {
     SplitGemm g;
     g.a = a_hi, g.a_lo = a_lo, g.w = w_hi, g.w_lo = w_lo, g.bias = bias, g.c = c, g.c_lo = c_lo;
     g.m_ptr = m_ptr, g.max_m = max_m, g.n = n, g.k = k;
-    g.weights_ready = weights_ready;
+    g.hints = hints;
     g.status_word = status_word;
     return launch_gemm_split(g, epilogue, plan, maps, stream);
   }
@@ -848,7 +844,7 @@ cudaError_t launch_gemm_tf32x3(const float* a_hi, const float* a_lo, const float
       !encode_2d_f32_sw128(&twh, w_hi, static_cast<uint64_t>(n), static_cast<uint64_t>(k), BN, maps) ||
       !encode_2d_f32_sw128(&twl, w_lo, static_cast<uint64_t>(n), static_cast<uint64_t>(k), BN, maps))
     return cudaErrorInvalidValue;
-  const int rev = reverse_m ? 1 : 0;
+  const int rev = reverse_m ? 1 : 0, rows_ready = hints.rows_ready ? 1 : 0;
   // The pair kernel needs enough 256 x 256 tiles at capacity to occupy the pairs; below that
   // the 128 x 128 tiles of the one-CTA kernel spread a small batch over more SMs.
   const long long pair_tiles = static_cast<long long>((max_m + BM2 - 1) / BM2) * (n / BN2);
@@ -860,7 +856,7 @@ cudaError_t launch_gemm_tf32x3(const float* a_hi, const float* a_lo, const float
       return cudaErrorInvalidValue;
 #define ETB_PAIR_CASE(E) \
   case E:                \
-    return launch_pair_epi<E>(tah, tal, twh, twl, twhh, twlh, bias, c, c_lo, m_ptr, max_m, n, k, status_word, rev, \
+    return launch_pair_epi<E>(tah, tal, twh, twl, twhh, twlh, bias, c, c_lo, m_ptr, max_m, n, k, status_word, rev, rows_ready, \
                               stream)
     switch (epilogue) {
       ETB_PAIR_CASE(kEpiNone);
@@ -874,7 +870,7 @@ cudaError_t launch_gemm_tf32x3(const float* a_hi, const float* a_lo, const float
   }
 #define ETB_CASE(E) \
   case E:           \
-    return launch_epi<E>(tah, tal, twh, twl, bias, c, c_lo, m_ptr, max_m, n, k, status_word, rev, stream)
+    return launch_epi<E>(tah, tal, twh, twl, bias, c, c_lo, m_ptr, max_m, n, k, status_word, rev, rows_ready, stream)
   switch (epilogue) {
     ETB_CASE(kEpiNone);
     ETB_CASE(kEpiBias);

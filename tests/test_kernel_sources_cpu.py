@@ -83,3 +83,15 @@ def test_what_is_in_flight_lands_even_when_a_role_has_given_up():
         body = attention[kernel]
         assert "drain_attention(bar_qk, qk_issued, bar_v, v_issued, bar_mma, mma_issued)" in body
         assert body.count("umma_commit(bar_mma);") == body.count("++mma_issued;") == 2
+
+
+def test_only_a_ready_row_count_is_read_in_front_of_the_wait():
+    """The row count may come in under the wait where the launch says so (rows_ready); nothing else that a kernel of
+    the pass writes may."""
+    helper = re.search(r"int pdl_wait_row_count\(.*?\n\}", open(os.path.join(CSRC, "common.cuh")).read(), re.S).group(0)
+    assert re.search(r"if \(ready != 0\) v = ld_row_count\(p\);\s*pdl_wait\(\);\s*if \(ready == 0\) v = ld_row_count", helper)
+    for name in FILES:
+        for kernel, _, body in kernels(read(name)):
+            for call in re.findall(r"[^;]*\bld_row_count\([^;]*;", body):
+                assert "rows_ready ?" in call, f"{name}: {kernel}: {call.strip()}"
+            assert not re.search(r"int M = \*m_ptr", body) or "pdl_wait()" not in body, f"{name}: {kernel}"
