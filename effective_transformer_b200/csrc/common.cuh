@@ -151,9 +151,9 @@ __device__ __forceinline__ Vec16 ld_activation_v4(const void* p) {
                : "memory");
   return v;
 }
-// The row count of a pass (*m_ptr, *t_ptr), from L2.  With `ready` it may be read in front of pdl_wait(): the kernel
-// that wrote it had completed before this kernel could be launched (see GemmHints).
-__device__ __forceinline__ int ld_row_count(const int* p) {
+// An int from L2.  In front of pdl_wait() only for what a kernel wrote that had completed, or had fenced its stores,
+// before this kernel could be launched: the row count of a pass (GemmHints), the attention plan.
+__device__ __forceinline__ int ld_l2_s32(const int* p) {
   int v;
   asm volatile("ld.relaxed.gpu.global.s32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
   return v;
@@ -161,9 +161,9 @@ __device__ __forceinline__ int ld_row_count(const int* p) {
 // pdl_wait() and the row count, clamped to [0, max_rows]; a count that is ready comes in under the wait.
 __device__ __forceinline__ int pdl_wait_row_count(const int* p, int max_rows, int ready) {
   int v = 0;
-  if (ready != 0) v = ld_row_count(p);
+  if (ready != 0) v = ld_l2_s32(p);
   pdl_wait();
-  if (ready == 0) v = ld_row_count(p);
+  if (ready == 0) v = ld_l2_s32(p);
   return v < 0 ? 0 : (v > max_rows ? max_rows : v);
 }
 // Through L2 only: for rows that other CTAs of the same kernel have just written.
@@ -429,20 +429,23 @@ cudaError_t launch_attention_tcgen05_long(const __half* q, const __half* k, cons
 // attr_mask given ([B, seq, seq], 1 = attend; with batch_idx / word_idx of the packed rows): a
 // general mask with the reference op's semantics (padded keys take part with K = V = 0).
 size_t attention_plan_ints(int batch, int max_tokens);
+// dependents_last: the plan is in L2 before a kernel behind this one can start (`plan_ready` below); otherwise they may
+// start while it is being made.
 cudaError_t launch_attention_plan(const int* cu_seqlens, int batch, int max_tokens, int* plan,
-                                  cudaStream_t stream);
+                                  cudaStream_t stream, bool dependents_last = false);
 // The same from the packed rows' sequence numbers; also writes cu_seqlens (as
 // launch_seq_bounds_from_batch_idx does).
 bool attention_plan_from_rows_supported(int batch, int max_tokens);
 cudaError_t launch_attention_plan_from_rows(const int* batch_idx, const int* t_ptr, int batch, int max_tokens,
-                                            int* cu_seqlens, int* plan, cudaStream_t stream);
+                                            int* cu_seqlens, int* plan, cudaStream_t stream,
+                                            bool dependents_last = false);
 cudaError_t launch_attention_tcgen05(const __half* q, const __half* k, const __half* v,
                                      long long token_stride, long long head_stride, __half* ctx,
                                      const int* plan, int batch, int max_tokens, int heads, int d,
                                      int* status_word, cudaStream_t stream, bool reverse = false,
                                      TensorMapCache* maps = nullptr, const __half* attr_mask = nullptr,
                                      const int* batch_idx = nullptr, const int* word_idx = nullptr, int seq = 0,
-                                     const uint32_t* mask_bits = nullptr);
+                                     const uint32_t* mask_bits = nullptr, bool plan_ready = false);
 // The general mask as bits per token, once per batch, for the launches of its layers (mask_bits above).
 constexpr int kMaskBitsBytes = 32;  // per token
 cudaError_t launch_attention_mask_bits(const __half* attr_mask, const int* batch_idx, const int* word_idx,

@@ -560,7 +560,8 @@ int run_layer(et_handle_t h, const LayerWeights& lw, const T* x_in, T* x_out, co
                                        reinterpret_cast<__half*>(ctx), ws.attn_plan, batch, max_m, heads, d,
                                        ws.status, s, turn(), &h->maps,
                                        static_cast<const __half*>(h->cur_attr_mask), h->cur_batch_idx,
-                                       h->cur_word_idx, seq, h->mask_bits_ready ? ws.mask_bits() : nullptr));
+                                       h->cur_word_idx, seq, h->mask_bits_ready ? ws.mask_bits() : nullptr,
+                                       true));
   else if (masked)
     ET_LAUNCH(h, ET_PROF_ATTENTION, 1, s,
               launch_attention_masked_simt<T>(qkv, qkv + hid, qkv + 2 * hid, 3LL * hid, d, ctx,
@@ -572,7 +573,8 @@ int run_layer(et_handle_t h, const LayerWeights& lw, const T* x_in, T* x_out, co
                                        reinterpret_cast<const __half*>(qkv) + hid,
                                        reinterpret_cast<const __half*>(qkv) + 2 * hid, 3LL * hid, d,
                                        reinterpret_cast<__half*>(ctx), ws.attn_plan, batch, max_m, heads, d,
-                                       ws.status, s, turn(), &h->maps));
+                                       ws.status, s, turn(), &h->maps, nullptr, nullptr, nullptr, 0, nullptr,
+                                       true));
   else if (tc)
     ET_LAUNCH(h, ET_PROF_ATTENTION, 1, s, launch_attention_tc(reinterpret_cast<const __half*>(qkv),
                                    reinterpret_cast<const __half*>(qkv) + hid,
@@ -786,7 +788,7 @@ int stack_impl(et_handle_t h, int batch, int seq, cudaStream_t s) {
   const bool tiles = h->cfg.dtype == ET_FP16 && !h->use_simt && seq <= 128 && max_m > 0;
   if (tiles)  // the packed-tile attention serves key-only and general masks
     ET_LAUNCH(h, ET_PROF_PADDING_OFFSETS, 1, s,
-              launch_attention_plan(ws.cu_seqlens, batch, max_m, ws.attn_plan, s));
+              launch_attention_plan(ws.cu_seqlens, batch, max_m, ws.attn_plan, s, true));
   if (tiles && h->cur_attr_mask != nullptr) {
     // (a row of stage_out is hidden * 2 bytes, 256 at least; a token's bits are 32)
     static_assert(kMaskBitsBytes <= 256, "the bits of a token must fit a row of stage_out");
@@ -1338,10 +1340,10 @@ int et_layer(et_handle_t h, int layer, const et_encoder_param_t* p, const et_tra
   if (one_kernel) {
     ET_LAUNCH(h, ET_PROF_PADDING_OFFSETS, 1, s,
               launch_attention_plan_from_rows(p->batch_idx, p->valid_word_num, batch, max_m, h->ws.cu_seqlens,
-                                              h->ws.attn_plan, s));
+                                              h->ws.attn_plan, s, true));
   } else if (tiles) {
     ET_LAUNCH(h, ET_PROF_PADDING_OFFSETS, 1, s,
-              launch_attention_plan(h->ws.cu_seqlens, batch, max_m, h->ws.attn_plan, s));
+              launch_attention_plan(h->ws.cu_seqlens, batch, max_m, h->ws.attn_plan, s, true));
   } else if (h->cur_attr_mask != nullptr) {
     ET_LAUNCH(h, ET_PROF_PADDING_OFFSETS, 1, s,
               launch_position_rows(p->batch_idx, p->word_idx, p->valid_word_num, batch, seq, h->ws.pos_row, s));
