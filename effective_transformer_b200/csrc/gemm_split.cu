@@ -526,17 +526,33 @@ bool encode_split(CUtensorMap* map, bool tf32, const void* base, int rows, int k
 //   out       64x4 426  64x2 460  - 467    64x4 490 - 542            64x2 526 - 555   64x2 591 - 608   64x2 733 - 707
 //   FFN1      64x2 425  64x4 471  - 460    64x2 488 - 504            64x2 561 - 517   64x1 638 - 592   - 706
 //   FFN2      64x8 425  64x4 489  - 638    64x8 489 64x4 525 - 647   64x4 530 - 660   64x2 587 - 660   64x2 707 - 734
-// and with every row of 2048 valid FFN2 64x2 919, - 839.  BERT-large at capacity 64: QKV 64x3 848, - 910; FFN1
-// 64x3 854, 64x2 890, - 900.  fp32, BERT-base, capacity 64 / 256 / 512:
+// and with every row of 2048 valid FFN2 64x2 919, - 839.  BERT-large fp16, capacity 128 / 256 / 512 / 768 / 1024 /
+// 1280 (55 to 65 % valid; the rule's plan first, then the best other one and the persistent kernels):
+//   QKV       64x3 944 64x5 927 - 980   - 1129 64x2 1115   - 1206 64x2 1226   - 1339   - 1441   - 1612
+//   out       64x5 939 64x4 921 - 1073   64x3 1127 64x5 1116 - 1250   64x3 1206 64x4 1199 - 1271
+//             64x2 1338 64x3 1314 - 1377   - 1441 64x2 1392   - 1611
+//   FFN1      64x3 943 - 988   - 1128 64x2 1144   - 1205   - 1340   - 1441   - 1611
+//   FFN2      64x8 939 - 1363   64x6 1127 - 1503   64x3 1206 64x4 1176 - 1502   64x2 1339 64x3 1289 - 1526
+//             64x2 1441 - 1625   - 1611 64x2 1416
+// It holds there, but stops early for K = 4096 (1536 rows: - 1664, 64x2 1530).  fp32, BERT-base, capacity 64 / 256 / 512:
 //   QKV       64x3 755  - 853              64x2 949 128x2 981 - 1001  128x2 1223 - 1170
 //   out       64x8 754  - 876              64x5 949 64x4 962 - 1064   128x5 1170 64x2 1173 - 1342
 //   FFN1      128x5 755 64x2 767 - 856     128x2 949 64x2 1005 - 965  128x2 1162 - 1155
 //   FFN2      64x8 755  - 1269             128x8 951 64x4 978 - 1401  128x5 1186 64x2 1295 - 1669
+// fp32, BERT-large, capacity 128 / 256 / 512: QKV 128x5 2175 64x2 2086 - 2217, 128x2 2666 - 2601, - 4048 128x2 3924; out
+// 64x6 2188 - 2529, 64x4 2665 - 2959, 128x4 4047 - 4191; FFN1 128x4 2177 64x2 2090 - 2293, - 2659, - 4046; FFN2 64x6
+// 2183 - 3470, 64x4 2668 - 3833, - 4047 128x6 3237 (384 rows: - 3899, 128x6 2730: its clusters are counted out below).
 // fp16: the most CTAs per tile with five 64-wide steps of K each to hide the load latency, or three where the grid
 // is small enough (two thirds of the SMs) not to share L2 bandwidth.  Two CTAs fit an SM, but clusters of more
 // than two stop finding places on a third more CTAs than SMs, and a short K does not pay for more either.
-// The projection in front of the attention gains least: up to one row tile only, and without a cluster where its
-// tiles leave three quarters of the SMs to the kernels around it.
+// The rule goes by capacity; a mostly empty batch pays for CTAs that find no rows.
+// The projection in front of the attention gains least: up to one row tile only, three CTAs per tile, none of them with
+// less than two steps of K (384, 6 steps: three 432 and 448, persistent 411 and 434).  us per pass at capacity 64 and
+// 128 with one / three CTAs / the persistent kernels, by hidden size:
+//   512   441 385 401,  481 435 439      640   513 483 481,  496 459 462      768   426 448 454,  447 470 474
+//   896   611 569 580,  652 607 603      1024  501 453 474,  572 517 526      1152  629 576 589,  646 598 600
+// One CTA without a cluster wins at 768 alone (with a feed-forward width of 2048 too: 393 423 420), by 5 %; why is not
+// known, so that line lies between the neighbours that were measured, K = 640 and 896.
 // fp32: one CTA fits an SM; among the plans whose clusters all find one the one whose CTA fetches the least, 64
 // or 48 KB per 32-wide step, a 128-wide tile's longer reduction counted as another 128 KB.  From six row tiles on a
 // third more CTAs than SMs is taken where K is long: a batch has padding, and the tiles it leaves empty cost next
@@ -550,9 +566,11 @@ static SplitPlan gemm_split_plan(int max_m, int n, int k, bool tf32, bool feeds_
   if (!tf32) {
     const long long tiles = m_tiles * (n / 64);
     if (n % 64 != 0 || (feeds_attention && m_tiles > 1)) return best;
-    if (feeds_attention && num_kb <= 12 && 8 * tiles > sms && 4 * tiles <= sms) {
-      best.splits = 1;
-      return best;
+    if (feeds_attention) {
+      if (num_kb < 8) return best;
+      if (num_kb > 10 && num_kb <= 12 && 4 * tiles <= sms) best.splits = 1;
+      else if (9 * tiles <= 4 * sms) best.splits = 3;
+      if (best.splits != 0) return best;
     }
     for (const int splits : kCounts) {
       const int share = num_kb / splits;

@@ -21,6 +21,8 @@ SPLIT_ROUTES = [
     ("fp16", 40, 256, 3072, 768, 2, (64, 2)),
     ("fp16", 639, 640, 1024, 4096, 4, (64, 2)),
     ("fp16", 64, 64, 3072, 1024, 1, (64, 3)),
+    ("fp16", 97, 128, 1536, 512, 1, (64, 3)),
+    ("fp16", 128, 128, 2688, 896, 1, (64, 3)),
     ("fp16", 2, 128, 4096, 1024, 2, (64, 3)),
     ("fp16", 385, 512, 1024, 1024, 4, (64, 3)),
     ("fp16", 512, 512, 1024, 4096, 4, (64, 3)),

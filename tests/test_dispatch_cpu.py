@@ -32,6 +32,15 @@ def test_large_batches_run_the_persistent_kernels(hidden, ffn):
             assert route("fp16", 64, n, k, epi_ln)[1] == 0
 
 
+@pytest.mark.parametrize("hidden,splits", [(256, 0), (384, 0), (512, 3), (640, 3), (768, 1), (896, 3), (1024, 3), (1152, 3)])
+def test_projection_in_front_of_the_attention_by_hidden_size(hidden, splits):
+    """One row tile: the plans as they were measured on both sides of each line; more rows, the persistent kernels."""
+    for epi in (1, 7):
+        for rows in (1, 64, 128):
+            assert route("fp16", rows, 3 * hidden, hidden, epi)[1] == splits
+        assert route("fp16", 129, 3 * hidden, hidden, epi)[1] == 0
+
+
 def test_invalid_shapes_are_refused():
     lib, a, b = _capi.load(), C.c_int(), C.c_int()
     for dtype, rows, n, k, epi in ((7, 8, 128, 64, 0), (0, 0, 128, 64, 0), (0, 8, 100, 64, 0), (0, 8, 128, 0, 0),
