@@ -641,8 +641,8 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_q, const __gri
 // tile streams in under the softmax and the second MMA, V under the read of O_j and the next scores.  What
 // bounds it is that phase chain (about 7 k cycles per key tile), hidden by the four CTAs of an SM; one CTA per
 // query tile instead of one per (sequence, head) shortens the longest chain from (len / 64)^2 steps to len / 128.
-// Measured under ncu, 32 sequences of 64 to 512 tokens, 12 heads: 43 us per launch, of which the issue slots are
-// busy 42 % and the exponential unit 36 %; attention_tc_kernel, a CTA per (sequence, head): 195 us.
+// Measured under ncu, 32 sequences of 64 to 512 tokens, 12 heads: 42 us per launch, of which the issue slots are
+// busy 41 % and the exponential unit 34 %; attention_tc_kernel, a CTA per (sequence, head): 195 us.
 // The grid is not persistent: CTAs differ by the sequence's length, and the hardware's order of starting them
 // balances that; those beyond a sequence's end leave at once.
 __global__ void __launch_bounds__(kThreads, kCtasPerSm)

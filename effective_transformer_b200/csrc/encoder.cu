@@ -129,7 +129,7 @@ inline size_t ln_counter_ints(size_t rows) { return round_up(rows, 256) / 32 + 8
 inline size_t ws_round(size_t bytes) { return round_up(bytes == 0 ? 16 : bytes, 256); }
 
 // The LayerNorm can be deferred into the projections around it (fp16 tensor-core path, every
-// projection on the CTA-pair kernel, statistics in 64-column pieces of rows of 128 * j columns).
+// projection on the CTA-pair or the split kernel, statistics in 64-column pieces of rows of 128 * j columns).
 bool defer_eligible(const et_config_t& c) {
   const int H = c.head_num * c.size_per_head;
   // rows of up to 1024 columns: the epilogues hold a row's partial sums in registers (width / 128 vectors)

@@ -1338,7 +1338,7 @@ cudaError_t launch_gemm_tcgen05(const __half* a, const __half* w_packed, const _
     lnp = *ln;
   }
   if (is_deferred_norm(epilogue)) {
-    // the pair kernel only; statistics in 64-column pieces of rows whose width is a multiple of 128
+    // the pair kernel and the split one; statistics in 64-column pieces of rows whose width is a multiple of 128
     if (ln == nullptr || (n % 256) != 0) return cudaErrorInvalidValue;
     const int width = epilogue == kEpiNormResidual ? n : k;  // of the tensor the statistics describe
     if ((width % 256) != 0 || width > 1024) return cudaErrorInvalidValue;
